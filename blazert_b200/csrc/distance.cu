@@ -39,13 +39,23 @@ __global__ void __launch_bounds__(kDistanceThreads)
   }
 }
 
-// Cylinders: the ellipse search takes 0 to 100 Newton steps per point (a quarter of random
-// points run all 100), so a warp of 32 fixed queries would idle most lanes while its slowest
-// one iterates.  Here each warp owns a contiguous range of queries and refills idle lanes from
-// it: every trip of the loop gives new queries to the idle lanes (their decisions before the
-// search, cylinder_setup) and one search step to the lanes in a search, all four sectors in
-// the same instructions.
-__global__ void __launch_bounds__(kDistanceThreads, 4)
+// Cylinders: the ellipse search takes 0 to about 25 Newton steps per point (8 on average, with
+// ellipse_search_step's cycle rule), so a warp of 32 fixed queries would idle lanes while its
+// slowest one iterates.  Here each warp owns a contiguous range of queries and refills idle
+// lanes from it: a trip of the loop gives new queries to the idle lanes (their decisions before
+// the search, cylinder_setup) and one search step to the lanes in a search, all four sectors
+// in the same instructions.
+//
+// A refill costs about two search steps whatever the number of lanes it fills, so it waits
+// until kRefillLanes are idle, and one wave of kCylinderBlocks resident blocks per SM gives
+// every warp the longest range (the last, partly idle trips of a range are paid once).
+// 1,048,576 points, all four kinds' passes together: refill at 1 / 8 / 16 / 24 / 32 idle lanes
+// 313 / 287 / 284 / 276 / 304 us on 8 blocks per SM; then 4 / 8 / 16 blocks per SM 270 / 276 /
+// 282 us, and 20 or 28 lanes at 4 blocks 272 and 270 us.  Bound by issue: about 250
+// instructions a step, a third of them FP64, in dependent divisions and square roots.
+constexpr int kRefillLanes = 24;
+constexpr int kCylinderBlocks = 4;
+__global__ void __launch_bounds__(kDistanceThreads, kCylinderBlocks)
     cylinder_distance_kernel(const SceneView S, const DistanceIO io) {
   const KindView &K = S.k[kCylinders];
   const unsigned full = 0xFFFFFFFFu;
@@ -60,7 +70,7 @@ __global__ void __launch_bounds__(kDistanceThreads, 4)
   CylinderQuery q;
   for (;;) {
     const unsigned idle = __ballot_sync(full, !busy);
-    if (idle && cursor < end) {
+    if (__popc(idle) >= kRefillLanes && cursor < end) {
       if (!busy) {
         const uint64_t j = cursor + __popc(idle & ((1u << lane) - 1u));
         if (j < end) {
@@ -151,7 +161,7 @@ cudaError_t launch_distance(const SceneView &S, int kind, const DistanceIO &io, 
       distance_kernel<kPlanes><<<grid, kDistanceThreads, 0, stream>>>(S, io);
       break;
     default:
-      cylinder_distance_kernel<<<grid, kDistanceThreads, 0, stream>>>(S, io);
+      cylinder_distance_kernel<<<grid_of(io.n, sms, kCylinderBlocks), kDistanceThreads, 0, stream>>>(S, io);
       break;
   }
   return cudaGetLastError();

@@ -75,6 +75,8 @@ BZR_HD double root_gap(double val, double s) {
   return (val * val > s * s) ? sqrt(val * val - s * s) : sqrt(s * s - val * val);
 }
 
+constexpr int kSearchSteps = 100;  // newton_iteration's step limit (cylinder.h:594-614)
+
 struct EllipseBranch {
   double A, B, X, Y, sg, tg;
 };
@@ -112,16 +114,38 @@ BZR_HD EllipseSearch ellipse_search(const EllipseBranch &e) {
 // then the nudge of a value that lands on |v| == a (the cylinder's a in every branch, as the
 // reference).  The derivative and the step take the same s = sqrt(|v^2 - A^2|), computed once.
 // Returns false when the loop ends (v is then final).
-BZR_HD bool ellipse_search_step(const EllipseSearch &S, double a, double &v, int &steps) {
+//
+// The step maps v to the next v and depends on nothing else, so a value that comes back makes
+// the rest of the search periodic: every further value, and whether its derivative ends the
+// loop (it did not the first time), is known.  Half of random points around a cylinder never
+// reach |R'| < 1e-7 -- the derivative's own rounding is larger -- and settle within 4 to 20
+// steps on a value (four in five of them) or on two to five neighbouring ones, then step on
+// them until the count reaches 100.  A step that returns its own argument therefore ends the
+// search with that value, and a value equal to the mark (`mark`, taken every 4 steps at
+// `mark_at`, every 16 after 24) lets the count skip all whole periods up to 100: the same final v, bit for bit,
+// for 8 steps in place of 53 on average.  Both compare bits, so that -0 and 0 stay apart.
+// B200, 1,048,576 points on 1,000 cylinders: 695 -> 195 us with the
+// kernel's refill rule (cylinder_distance_kernel).
+BZR_HD bool ellipse_search_step(const EllipseSearch &S, double a, double &v, int &steps,
+                                double &mark, int &mark_at) {
   const EllipseBranch &e = S.e;
   const double s = root_gap(v, e.A);
   const double d = -2 * (e.X - v) - S.B2 * v * (S.BA * s - e.tg * e.Y) / (e.A * s);
-  if (!((fabs(d) >= 1e-7) && (steps < 100))) return false;
+  if (!((fabs(d) >= 1e-7) && (steps < kSearchSteps))) return false;
   const double num = (S.A3X - e.sg * (e.A * v * v * e.X)) * s + e.B * v * v * v * e.Y;
   const double den = (S.D0 - e.sg * (e.A * v * v) + e.sg * (S.BB * v * v / e.A)) * s + S.AABY;
+  const double last = v;
   v = num / den;
   ++steps;
   if (fabs(v) == a) v += kDblEps;
+  if (dbits(v) == dbits(last)) return false;
+  if (dbits(v) == dbits(mark)) {
+    const int period = steps - mark_at;
+    steps += (kSearchSteps - steps) / period * period;
+  } else if ((steps & (steps < 24 ? 3 : 15)) == 0) {
+    mark = v;
+    mark_at = steps;
+  }
   return true;
 }
 
@@ -150,8 +174,9 @@ BZR_HD double ellipse_distance(double a, double b, double xq, double yq) {
   const EllipseSearch S = ellipse_search(ellipse_branch(a, b, xq, yq));
   const double percentage = 0.95;
   double v = S.e.X > 0 ? percentage * S.e.A : -percentage * S.e.A;
-  int steps = 0;
-  while (ellipse_search_step(S, a, v, steps)) {
+  double mark = v;
+  int steps = 0, mark_at = 0;
+  while (ellipse_search_step(S, a, v, steps, mark, mark_at)) {
   }
   return ellipse_finish(S.e, v);
 }
@@ -167,6 +192,8 @@ struct CylinderQuery {
   double top = 0.0, bottom = 0.0;
   int region = 0;       // 0 result ready; 1 inside; 2 beside the shell; 3 outside above/below
   int steps = 0;        // search steps taken
+  double mark = 0.0;    // a value of the search and the step it was taken at, to see a
+  int mark_at = 0;      // value come back (ellipse_search_step)
   double result = 0.0;
 };
 
@@ -212,6 +239,7 @@ BZR_HD CylinderQuery cylinder_setup(D3 c, double a, double b, double height, con
   q.S = ellipse_search(ellipse_branch(a, b, x_q, y_q));
   const double percentage = 0.95;
   q.v = q.S.e.X > 0 ? percentage * q.S.e.A : -percentage * q.S.e.A;
+  q.mark = q.v;
   return q;
 }
 
@@ -226,7 +254,7 @@ BZR_HD double cylinder_finish(const CylinderQuery &q, double v) {
 
 // One pass of the search's loop for a query in its search: false when it has ended.
 BZR_HD bool cylinder_search_step(CylinderQuery &q) {
-  return ellipse_search_step(q.S, q.a, q.v, q.steps);
+  return ellipse_search_step(q.S, q.a, q.v, q.steps, q.mark, q.mark_at);
 }
 
 // cylinder.h:677-759
