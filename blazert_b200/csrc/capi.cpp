@@ -40,12 +40,12 @@ int cuda_fail(cudaError_t e, const char *what) {
 // Allocations left before the injected failure (bzr_debug_fail_allocation); 0: none armed.
 std::atomic<int64_t> g_alloc_countdown{0};
 
-// Per-call device words: kSlots slots of kSlotWords = {launch_trace's counters
-// (kTraceCounterWords), error word, 3 spare}; one sticky error word for device-array calls
+// Per-call device words: kSlots slots of kSlotWords = launch_trace's words (kTraceWords), whose
+// word kTraceCounterWords is the call's error word; one sticky error word for device-array calls
 // follows the slots.
 constexpr int kSlots = 256;
-constexpr int kSlotWords = 16;
-static_assert(bzr::kTraceCounterWords + 4 <= kSlotWords, "slot layout");
+constexpr int kSlotWords = (bzr::kTraceWords + 15) / 16 * 16;
+static_assert(bzr::kTraceCounterWords < bzr::kTraceListWord, "slot layout");
 constexpr int kStickyWord = kSlots * kSlotWords;
 // Host-array batches: split into at most host_chunks (default kHostChunks, at most kMaxChunks)
 // chunks of at least host_min_chunk (default kMinChunk) rays.
@@ -572,6 +572,8 @@ static int run_small(bzr_scene *s, size_t n, const double *org, const double *di
   for (int k = 0; k < bzr::kNumKinds; ++k) {
     plan.blocks[k] = std::max(1, std::min(plan.blocks[k], need_blocks));
     plan.blocks32[k] = std::max(1, std::min(plan.blocks32[k], need_blocks));
+    plan.blocks64w[k] = std::max(1, std::min(plan.blocks64w[k], need_blocks));
+    plan.blocks_rest[k] = std::max(1, std::min(plan.blocks_rest[k], need_blocks));
   }
   cudaError_t e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = bzr::launch_trace(s->view, ci, mode, plan, st, counters, totals);
@@ -715,6 +717,8 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
   for (int k = 0; k < bzr::kNumKinds; ++k) {
     chunk_plan.blocks[k] = std::max(1, chunk_plan.blocks[k] / s->host_grid_div);
     chunk_plan.blocks32[k] = std::max(1, chunk_plan.blocks32[k] / s->host_grid_div);
+    chunk_plan.blocks64w[k] = std::max(1, chunk_plan.blocks64w[k] / s->host_grid_div);
+    chunk_plan.blocks_rest[k] = std::max(1, chunk_plan.blocks_rest[k] / s->host_grid_div);
   }
   cudaError_t e = cudaSuccess;
   for (size_t c = 0; c < nchunks && e == cudaSuccess; ++c) {

@@ -28,7 +28,9 @@
 //    std::min argument order (blazert/bvh/intersect.h:33-51).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "alloc.h"
 #include "layout.h"
@@ -76,21 +78,25 @@ __device__ __forceinline__ void init_stack(Stack &sk, uint32_t &tid, uint32_t ca
 // flush), and then every dependent node fetch of the first rays waits for DRAM.  The grid
 // first asks L2 for the breadth-first prefix of the node array (the top levels every ray
 // visits) and for the leaf-ordered primitive data, at most kPrefetchBytes of each, one
-// 128-byte line per thread per round.  A hint only: nothing waits for it.
+// 128-byte line per thread per round.  A hint only: nothing waits for it.  A small batch's grid
+// does not go round for more than kPrefetchRounds: its few rays need less than the loop costs
+// (one block over 4 MB is 256 rounds before its first ray).
 constexpr size_t kPrefetchBytes = size_t(4) << 20;
+constexpr size_t kPrefetchRounds = 2;
 
 __device__ __forceinline__ void prefetch_l2(const void *base, size_t bytes) {
   if (!base) return;
   bytes = bytes < kPrefetchBytes ? bytes : kPrefetchBytes;
   const size_t step = size_t(gridDim.x) * blockDim.x * 128;
+  bytes = bytes < kPrefetchRounds * step ? bytes : kPrefetchRounds * step;
   for (size_t off = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 128; off < bytes;
        off += step)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char *>(base) + off));
 }
 
-template <int KIND, bool MIXED>
+template <int KIND, bool WIDE>
 __device__ __forceinline__ void prefetch_kind(const KindView &K) {
-  if (MIXED && K.mixed_ok) {  // the wide image: nodes, then leaf records (and vertices)
+  if (WIDE && K.mixed_ok) {  // the wide image: nodes, then leaf records (and vertices)
     prefetch_l2(K.wide, size_t(K.n_wide) * kWideBytes);
     prefetch_l2(K.leaves, size_t(K.n_leaf16) * 16);
     if (KIND == kMesh) prefetch_l2(K.verts, size_t(K.n_verts) * kVertexDoubles * sizeof(double));
@@ -121,15 +127,24 @@ __device__ __forceinline__ void griddep_wait() {
 
 // One kind over the whole batch.  first: this pass writes the whole output record.
 // COUNT: also sums the work counters into totals[16] (per kind: box tests, primitive tests,
-// node fetches, leaf fetches; see Counts).  MIXED: the rays the FP32 test covers walk the wide
-// image; the others are appended to io.defer for the FP64 pass that follows (cylinders always
-// take the FP64 traversal).  Keeping the FP64 walk out of the wide kernel keeps its registers
-// for the wide walk.  io.n_dev: the FP64 pass over a deferred list reads its ray count there.
-template <int KIND, bool COUNT, bool MIXED, bool LOCAL>
+// node fetches, leaf fetches; see Counts).  F: NoWalk, the binary FP64 traversal; RayW or RayD,
+// the wide walk in FP32 or FP64, which hands on the rays that it does not cover (f.ok) or that
+// end it without a result (kRedoLeaf); Rest, the binary traversal of those (cylinders always
+// take the binary traversal).  Keeping the binary walk out of the wide kernel keeps its
+// registers for the wide walk.
+struct NoWalk {
+  using Bound = float;
+};
+struct Rest {
+  using Bound = float;
+};
+
+template <int KIND, bool COUNT, class F, bool LOCAL>
 __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO &io, int first,
                                                 uint32_t *work_counter,
                                                 unsigned long long *totals) {
-  constexpr bool kWide = MIXED && KIND != kCylinders;
+  constexpr bool kRest = std::is_same<F, Rest>::value;
+  constexpr bool kWide = !std::is_same<F, NoWalk>::value && !kRest && KIND != kCylinders;
   // The next kernel on the stream may be scheduled now: it waits (griddep_wait) for this grid
   // to complete before it reads anything this grid writes.
   griddep_launch_dependents();
@@ -140,8 +155,8 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
   uint32_t tid;
   init_stack<LOCAL>(sk, tid, S.stack_cap, smem, lkey, lref);
   const KindView &K = S.k[KIND];
-  // (a deferred list is short: its pass leaves L2 to the rays)
-  if (!COUNT && !io.n_dev) prefetch_kind<KIND, kWide>(K);
+  // (the rays handed on are few as a rule: their pass leaves L2 to the rays)
+  if (!COUNT && !kRest) prefetch_kind<KIND, kWide>(K);
   // The first io.top_nodes nodes of the array this kernel walks (the top levels every ray
   // visits) are staged in shared memory after the stack.
   {
@@ -156,19 +171,31 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
     sk.n_top = n_top;
   }
   // Up to here only the scene was read; the counters, the rays' closest distances and the
-  // deferred list come from earlier kernels of the stream.
+  // lists come from earlier kernels of the stream.
   griddep_wait();
-  const uint32_t n = io.n_dev ? *io.n_dev : io.n;
-  if (n == 0) return;  // the same for every thread of the grid
+  // The rays of a Rest pass: the listed ones, or every ray that the wide walk does not cover
+  // when they outgrew their list, or every ray when those to redo outgrew theirs (a ray the
+  // wide walk has finished gives the same result again).
+  uint32_t n = io.n, n_uncovered = 0;
+  bool scan = false, all = false;
+  if constexpr (kRest) {
+    n_uncovered = *io.uncovered_count;
+    const uint32_t n_redo = *io.redo_count;
+    all = n_redo > kRedoList;
+    scan = all || n_uncovered > kUncoveredList;
+    n = all ? io.n : scan ? io.n + n_redo : n_uncovered + n_redo;
+    if (n == 0) return;  // the same for every thread of the grid
+  }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
   uint32_t pool_next = 0, pool_end = 0;  // warp-uniform
   bool exhausted = false;                // warp-uniform
+  bool list_full = false;                // warp-uniform: the list of uncovered rays is full
   bool active = false;
   uint32_t i = 0;
   Ray r;
-  RayW f;
-  float hl = 0.0f;
+  F f;
+  typename F::Bound hl = 0;
   KState st;
   Trav tv;
   Counts cnt = {};
@@ -190,22 +217,38 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
           const uint32_t rank = __popc(idle & below);
           const uint32_t idx = rank < avail ? pool_next + rank : base + (rank - avail);
           if (idx < n) {
-            i = io.perm ? io.perm[idx] : idx;
+            if constexpr (kRest) {
+              const uint32_t rays = scan ? io.n : n_uncovered;
+              i = idx >= rays ? io.redo[idx - rays]
+                  : !scan     ? io.uncovered[idx]
+                  : io.perm   ? io.perm[idx]
+                              : idx;
+            } else {
+              i = io.perm ? io.perm[idx] : idx;
+            }
             active = true;
             r = make_ray(io.org + 3 * size_t(i), io.dir + 3 * size_t(i),
                          io.tmin ? io.tmin[i] : 0.0, io.tmax ? io.tmax[i] : kDblMax);
             r.any_hit = io.any_hit != 0;
             if constexpr (kWide) {
-              f = make_ray_w(r);
+              f = make_ray_f(r, static_cast<const F *>(nullptr));
               if (K.mixed_ok && f.ok) {
                 wtrav_begin<KIND, COUNT>(K, r, f, st, hl, tv, &cnt);
               } else {
-                io.defer[atomicAdd(io.defer_count, 1u)] = i;
                 active = false;
                 deferred = true;
               }
             } else {
-              trav_begin<KIND, COUNT>(K, r, st, tv, &cnt);
+              if constexpr (kRest) {  // the wide walk has traced the rays it covers
+                if (scan && !all && idx < io.n &&
+                    (io.wide_mode == kModeMixed
+                         ? make_ray_f(r, static_cast<const RayW *>(nullptr)).ok
+                         : make_ray_f(r, static_cast<const RayD *>(nullptr)).ok)) {
+                  active = false;
+                  deferred = true;
+                }
+              }
+              if (active) trav_begin<KIND, COUNT>(K, r, st, tv, &cnt);
             }
           }
         }
@@ -217,21 +260,46 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
           pool_next += want;
         }
       }
-      if (!kWide || !__any_sync(kFull, deferred)) break;
+      if constexpr (!kWide && !kRest) break;
+      const unsigned handed = __ballot_sync(kFull, deferred);
+      if (!handed) break;
+      if constexpr (kWide) {
+        if (!list_full) {
+          uint32_t at = 0;
+          if (lane == 0) at = atomicAdd(io.uncovered_count, __popc(handed));
+          at = __shfl_sync(kFull, at, 0);
+          list_full = at + __popc(handed) > kUncoveredList;
+          at += __popc(handed & below);
+          if (deferred && at < kUncoveredList) io.uncovered[at] = i;
+        }
+      }
     }
     // every lane idle: the global counter has passed the end of the batch
     if (!__any_sync(kFull, active)) break;
     if (active) {
       if constexpr (kWide) {
-        if (tv.live) wtrav_to_leaf<KIND, COUNT>(K, f, hl, tv, sk, tid, io.error_word, &cnt);
+        if (tv.live) wtrav_to_leaf<KIND, COUNT>(K, r, f, hl, tv, sk, tid, io.error_word, &cnt);
+        // what only the leaf steps read of the ray is formed again here, so that no register
+        // holds it through the walk (1 / w has w's sign for a covered ray)
+        r.tmin = io.tmin ? ldg(io.tmin + i) : 0.0;
+        r.any_hit = io.any_hit != 0;
+        r.sx = f.oct & 1u, r.sy = (f.oct >> 1) & 1u, r.sz = f.oct >> 2;
         while (tv.live && tv.post != kNoLeaf)
-          wtrav_leaf<KIND, COUNT>(K, r, f, st, hl, tv, sk, tid, io.error_word, &cnt);
+          wtrav_leaf<KIND, COUNT>(K, r, f, st, hl, tv, io.error_word, &cnt);
+        if (!tv.live && tv.post == kRedoLeaf) {  // rare: the binary pass traces this ray
+          const uint32_t at = atomicAdd(io.redo_count, 1u);
+          if (at < kRedoList) io.redo[at] = i;
+          active = false;
+        }
       } else {
         if (tv.live) trav_to_leaf<KIND, COUNT>(K, r, st, tv, sk, tid, io.error_word, &cnt);
         if (tv.live) trav_leaf<KIND, COUNT>(K, r, st, tv, sk, tid, io.error_word, &cnt);
       }
-      if (!tv.live) {
-        if constexpr (kWide) wtrav_end<KIND>(K, r, st);
+      if (active && !tv.live) {
+        if constexpr (kWide) {
+          r.tmax = io.tmax ? ldg(io.tmax + i) : kDblMax;
+          wtrav_end<KIND>(K, r, st);
+        }
         finalize_kind<KIND>(S, r, st, i, first != 0, io.t, io.uv, io.normal, io.prim, io.geom,
                             io.hit);
         active = false;
@@ -256,7 +324,7 @@ template <int KIND, bool COUNT, bool LOCAL>
 __global__ void __launch_bounds__(kMaxTraceThreads)
     trace_kind_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
                       unsigned long long *totals) {
-  trace_kind_body<KIND, COUNT, false, LOCAL>(S, io, first, work_counter, totals);
+  trace_kind_body<KIND, COUNT, NoWalk, LOCAL>(S, io, first, work_counter, totals);
 }
 
 #ifndef BZR_WIDE_REGS
@@ -266,7 +334,27 @@ template <int KIND, bool COUNT, bool LOCAL>
 __global__ void __maxnreg__(BZR_WIDE_REGS)
     trace_wide_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
                       unsigned long long *totals) {
-  trace_kind_body<KIND, COUNT, true, LOCAL>(S, io, first, work_counter, totals);
+  trace_kind_body<KIND, COUNT, RayW, LOCAL>(S, io, first, work_counter, totals);
+}
+
+// The FP64 mode's wide walk, with the thread-local stack (other stacks take the binary walk).
+// Its cap of 80 registers (6 blocks of 128 per SM) is the measured optimum over the workloads:
+// terrain / mixed primitives / icosphere 4,415 / 1,394 / 99 us at 72, 4,606 / 1,387 / 94 at 80,
+// 4,964 / 1,417 / 105 at 88, 4,943 / 1,407 / 104 at 96.
+constexpr int kWide64Regs = 80;
+template <int KIND>
+__global__ void __maxnreg__(kWide64Regs)
+    trace_wide64_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
+                        unsigned long long *totals) {
+  trace_kind_body<KIND, false, RayD, true>(S, io, first, work_counter, totals);
+}
+
+// The binary pass over the rays that a wide pass handed on.
+template <int KIND, bool COUNT, bool LOCAL>
+__global__ void __launch_bounds__(kMaxTraceThreads)
+    trace_rest_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
+                      unsigned long long *totals) {
+  trace_kind_body<KIND, COUNT, Rest, LOCAL>(S, io, first, work_counter, totals);
 }
 
 template <int KIND, bool COUNT, bool MIXED, bool LOCAL>
@@ -354,7 +442,7 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
                        io.tmax ? io.tmax[i] : kDblMax);
           r.any_hit = io.any_hit != 0;
           if constexpr (kWide) {
-            f = make_ray_w(r);
+            f = make_ray_f(r, static_cast<const RayW *>(nullptr));
             use32 = K->mixed_ok && f.ok;
           }
           if (kWide && use32)
@@ -379,9 +467,13 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
     if (!__any_sync(kFull, active)) break;
     if (active) {
       if (kWide && use32) {
-        if (tv.live) wtrav_to_leaf<KIND, false>(*K, f, hl, tv, sk, tid, io.error_word, &cnt);
+        if (tv.live) wtrav_to_leaf<KIND, false>(*K, r, f, hl, tv, sk, tid, io.error_word, &cnt);
         while (tv.live && tv.post != kNoLeaf)
-          wtrav_leaf<KIND, false>(*K, r, f, st, hl, tv, sk, tid, io.error_word, &cnt);
+          wtrav_leaf<KIND, false>(*K, r, f, st, hl, tv, io.error_word, &cnt);
+        if (!tv.live && tv.post == kRedoLeaf) {  // rare: the binary walk, from the start
+          use32 = false;
+          trav_begin<KIND, false>(*K, r, st, tv, &cnt);
+        }
       } else {
         if (tv.live) trav_to_leaf<KIND, false>(*K, r, st, tv, sk, tid, io.error_word, &cnt);
         if (tv.live) trav_leaf<KIND, false>(*K, r, st, tv, sk, tid, io.error_word, &cnt);
@@ -510,11 +602,16 @@ inline bool use_local(const SceneView &S, const LaunchPlan &plan) {
   return !plan.shared_stack && S.stack_cap <= kLocalStack;
 }
 
-// Whether a pass of KIND in `mode` walks the wide image (and defers the rays it cannot).
+// Whether a pass of KIND in `mode` over n rays walks the wide image (and defers the rays it
+// cannot).  The FP64 mode does with the thread-local stack, from kWide64MinRays rays on; its
+// counting kernels count the binary walk.  Below, the launch of the pass over the deferred rays
+// (2 to 3 us a kind) costs more than the walk saves: one ray on an icosphere 12.2 us binary,
+// 15.5 wide; 32 rays 44.3 and 40.4, and through three kinds 183 and 131 us.
+constexpr uint32_t kWide64MinRays = 32;
 template <int KIND>
-bool walks_wide(const SceneView &S, int mode) {
-  return mode == kModeMixed && KIND != kCylinders && S.k[KIND].present && S.k[KIND].n_prims &&
-         S.k[KIND].mixed_ok;
+bool walks_wide(const SceneView &S, int mode, const LaunchPlan &plan, bool count, uint32_t n) {
+  return KIND != kCylinders && S.k[KIND].present && S.k[KIND].n_prims && S.k[KIND].mixed_ok &&
+         (mode == kModeMixed || (use_local(S, plan) && !count && n >= kWide64MinRays));
 }
 
 using TraceFn = void (*)(SceneView, RayIO, int, uint32_t *, unsigned long long *);
@@ -550,21 +647,34 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
   const bool early = after_trace && plan.early_launch;
   const TraceFn fp64 = local ? trace_kernel<KIND, false, false, true>()
                              : trace_kernel<KIND, COUNT, false, false>();
-  if (!walks_wide<KIND>(S, mode))
-    return launch_one(fp64, plan.blocks[KIND], th, smem, stream, early, S, io, first,
-                      counters + KIND, totals);
-  const TraceFn wide_fn = local ? trace_kernel<KIND, false, true, true>()
-                                : trace_kernel<KIND, COUNT, true, false>();
-  RayIO wide = io;
-  wide.defer_count = counters + kNumKinds + KIND;
-  RayIO rest = io;
-  rest.perm = io.defer;  // ray indices
-  rest.n_dev = wide.defer_count;
-  const cudaError_t e = launch_one(wide_fn, plan.blocks32[KIND], th, smem, stream, early, S,
-                                   wide, first, counters + KIND, totals);
-  if (e != cudaSuccess) return e;
-  return launch_one(fp64, plan.blocks[KIND], th, smem, stream, plan.early_launch, S, rest, first,
-                    counters + 2 * kNumKinds + KIND, totals);
+  // no more blocks than the batch fills
+  auto grid = [&](int blocks) {
+    return int(std::min<uint64_t>(uint64_t(blocks), (uint64_t(io.n) + th - 1) / th));
+  };
+  if constexpr (KIND != kCylinders) {
+    if (walks_wide<KIND>(S, mode, plan, COUNT, io.n)) {
+      const bool mixed = mode == kModeMixed;
+      const TraceFn wide_fn = !mixed ? trace_wide64_kernel<KIND>
+                              : local ? trace_kernel<KIND, false, true, true>()
+                                      : trace_kernel<KIND, COUNT, true, false>();
+      const TraceFn rest_fn = local ? trace_rest_kernel<KIND, false, true>
+                                    : trace_rest_kernel<KIND, COUNT, false>;
+      RayIO wide = io;
+      wide.uncovered_count = counters + 2 * kNumKinds + KIND;
+      wide.redo_count = counters + 3 * kNumKinds + KIND;
+      wide.uncovered = counters + kTraceListWord;
+      wide.redo = wide.uncovered + kUncoveredList;
+      wide.wide_mode = mode;
+      const cudaError_t e =
+          launch_one(wide_fn, grid(mixed ? plan.blocks32[KIND] : plan.blocks64w[KIND]), th, smem,
+                     stream, early, S, wide, first, counters + KIND, totals);
+      if (e != cudaSuccess) return e;
+      return launch_one(rest_fn, grid(plan.blocks_rest[KIND]), th, smem, stream,
+                        plan.early_launch, S, wide, first, counters + kNumKinds + KIND, totals);
+    }
+  }
+  return launch_one(fp64, grid(plan.blocks[KIND]), th, smem, stream, early, S, io, first,
+                    counters + KIND, totals);
 }
 
 // Resident blocks per SM of `fn` with `threads` per block and `smem` bytes of dynamic shared
@@ -594,18 +704,27 @@ cudaError_t prepare_kind(const SceneView &S, LaunchPlan *plan) {
     const cudaError_t e = grid_for(fn, th, smem, plan->sms, &ignored);
     if (e != cudaSuccess) return e;
   }
-  int *blocks = &plan->blocks[KIND], *blocks32 = &plan->blocks32[KIND];
-  if (use_local(S, *plan)) {
-    const cudaError_t e = grid_for(
-        reinterpret_cast<const void *>(trace_kernel<KIND, false, false, true>()), th,
-        smem_local, plan->sms, blocks);
-    if (e != cudaSuccess) return e;
-    return grid_for(reinterpret_cast<const void *>(trace_kernel<KIND, false, true, true>()), th,
-                    smem_local, plan->sms, blocks32);
-  }
-  const cudaError_t e = grid_for(shared_fns[0], th, smem, plan->sms, blocks);
+  const bool local = use_local(S, *plan);
+  const size_t bytes = local ? smem_local : smem;
+  cudaError_t e = grid_for(
+      local ? reinterpret_cast<const void *>(trace_kernel<KIND, false, false, true>())
+            : shared_fns[0], th, bytes, plan->sms, &plan->blocks[KIND]);
   if (e != cudaSuccess) return e;
-  return grid_for(shared_fns[2], th, smem, plan->sms, blocks32);
+  e = grid_for(local ? reinterpret_cast<const void *>(trace_kernel<KIND, false, true, true>())
+                     : shared_fns[2], th, bytes, plan->sms, &plan->blocks32[KIND]);
+  if constexpr (KIND != kCylinders) {
+    const void *rest_fns[2] = {reinterpret_cast<const void *>(trace_rest_kernel<KIND, true, false>),
+                               reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, false>)};
+    for (const void *fn : rest_fns)
+      if (e == cudaSuccess) e = grid_for(fn, th, smem, plan->sms, &plan->blocks_rest[KIND]);
+    if (local && e == cudaSuccess)
+      e = grid_for(reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, true>), th, bytes,
+                   plan->sms, &plan->blocks_rest[KIND]);
+    if (local && e == cudaSuccess)
+      e = grid_for(reinterpret_cast<const void *>(trace_wide64_kernel<KIND>), th, bytes, plan->sms,
+                   &plan->blocks64w[KIND]);
+  }
+  return e;
 }
 
 }  // namespace
@@ -653,20 +772,13 @@ cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const La
   RayIO sorted = io;
   sorted.chunk = plan.chunk;
   sorted.top_nodes = plan.top_nodes;
-  sorted.n_dev = nullptr;
-  // scratch from the pool: the sort's keys, permutation and bucket counts, then the deferred
-  // list of the wide passes unless the caller gave one
+  // scratch from the pool: the sort's keys, permutation and bucket counts
   const bool sort = plan.sort.enabled && io.n >= plan.sort_min_rays && trace_passes(S) > 0;
-  const bool defer = !io.defer && (walks_wide<kMesh>(S, mode) || walks_wide<kSpheres>(S, mode) ||
-                                   walks_wide<kPlanes>(S, mode));
   const size_t nb = size_t(1) << kSortBits;
-  const size_t sort_words = sort ? 2 * size_t(io.n) + nb : 0;
   uint32_t *scratch = nullptr;
-  if (sort || defer) {
-    e = bzr::pool_malloc(&scratch, (sort_words + (defer ? io.n : 0)) * sizeof(uint32_t),
-                         plan.pool, stream);
+  if (sort) {
+    e = bzr::pool_malloc(&scratch, (2 * size_t(io.n) + nb) * sizeof(uint32_t), plan.pool, stream);
     if (e != cudaSuccess) return e;
-    if (defer) sorted.defer = scratch + sort_words;
   }
   if (sort) {
     uint32_t *keys = scratch, *perm = scratch + io.n, *counts = scratch + 2 * size_t(io.n);

@@ -14,10 +14,16 @@ constexpr int kMaxTraceThreads = 256;  // largest block the trace kernels are co
 constexpr uint32_t kRayChunk = 32;     // default rays a warp takes from the global counter
 constexpr int kModeFp64 = 0;   // BZR_MODE_FP64
 constexpr int kModeMixed = 1;  // BZR_MODE_MIXED
-// Device words launch_trace takes per call: the work counter of each kind's pass, then for
-// each kind the count of rays its mixed pass deferred and the work counter of the FP64 pass
-// over them.
-constexpr int kTraceCounterWords = 3 * kNumKinds;
+// Device words launch_trace takes per call.  First kTraceCounterWords zeroed words: the work
+// counter of each kind's pass, then for each kind the work counter of the binary pass over the
+// rays its wide walk handed on, the count of those it did not cover and the count of those whose
+// walk ended without a result.  From kTraceListWord on, the first kUncoveredList and kRedoList
+// of these rays' indices (the kinds' passes use them one after the other).  Words in between
+// belong to the caller.
+constexpr int kTraceCounterWords = 4 * kNumKinds;
+constexpr int kTraceListWord = kTraceCounterWords + 4;
+constexpr uint32_t kUncoveredList = 96, kRedoList = 32;
+constexpr int kTraceWords = kTraceListWord + int(kUncoveredList + kRedoList);
 
 // Device pointers of one batch.  tmin / tmax may be null (0 and DBL_MAX); each output except t
 // may be null.  error_word collects kErr* bits.
@@ -39,12 +45,14 @@ struct RayIO {
   uint32_t chunk = kRayChunk;      // rays a warp takes per fetch: 32, 64, 128, or 0 for
                                    // exactly the lanes that are idle
   uint32_t top_nodes = 0;          // top-level nodes each block stages in shared memory
-  // Mixed-precision passes: rays the FP32 walk does not cover are appended to defer (one
-  // word per ray of the batch, or null for launch_trace to take it from plan.pool) and traced
-  // by an FP64 pass over that list right after.  Set by launch_trace.
-  uint32_t *defer = nullptr;
-  uint32_t *defer_count = nullptr;
-  const uint32_t *n_dev = nullptr;  // when set, the pass's ray count is *n_dev (not n)
+  // Wide passes: the rays the wide walk does not cover, or whose walk ends without a result,
+  // are counted here and the first of each noted in the lists, for the binary pass right after.
+  // A batch has few such rays or (axis-parallel ones) many: a short list that needs no
+  // allocation serves the few, and past it the binary pass looks at every ray again.  Set by
+  // launch_trace.
+  uint32_t *uncovered_count = nullptr, *redo_count = nullptr;
+  uint32_t *uncovered = nullptr, *redo = nullptr;
+  int wide_mode = 0;  // the mode whose wide pass handed the rays on (its cover test)
 };
 
 // Coherence sort of a batch: rays are processed in the order of a 32-bit key -- the direction
@@ -70,6 +78,8 @@ struct LaunchPlan {
   bool early_launch = true;
   int blocks[kNumKinds] = {0, 0, 0, 0};    // FP64 kernels
   int blocks32[kNumKinds] = {0, 0, 0, 0};  // mixed-precision kernels
+  int blocks64w[kNumKinds] = {0, 0, 0, 0};  // the FP64 mode's wide kernels
+  int blocks_rest[kNumKinds] = {0, 0, 0, 0};  // the binary passes after wide ones
   RaySort sort;
   uint32_t sort_min_rays = 1u << 16;  // smaller batches are traced in their own order
   cudaMemPool_t pool = nullptr;       // stream-ordered scratch (keeps its memory mapped)
@@ -140,14 +150,13 @@ int trace_passes(const SceneView &S);
 // be non-null when trace_passes(S) > 1 (it carries the closest distance between passes).
 // When plan.sort.enabled and the batch has at least plan.sort_min_rays rays, a coherence sort
 // runs first (scratch from plan.pool, stream-ordered).
-// counters: kTraceCounterWords device words, zeroed here.  totals (device, 8 x uint64, or
-// null): when given, the counting kernels add per kind the box tests (totals[0..3]) and
+// counters: kTraceWords device words, zeroed here as far as needed.  totals (device, 8 x uint64,
+// or null): when given, the counting kernels add per kind the box tests (totals[0..3]) and
 // primitive tests (totals[4..7]) of every ray.
-// A mixed-precision pass of a kind whose wide image exists is two kernels: the wide walk over
-// the batch, which appends the rays its FP32 test does not cover (a direction component of 0
-// or below 2^-40 in magnitude, an origin coordinate or tmin beyond 1e18, NaN) to io.defer,
-// then the FP64 walk over that list.  io.defer may carry io.n words of scratch; null takes
-// them from plan.pool.
+// A pass of a kind whose wide image exists is two kernels: the wide walk over the batch, which
+// hands on the rays it does not cover (FP32: a direction component of 0 or below 2^-40 in
+// magnitude, an origin coordinate or tmin beyond 1e18, NaN; FP64: RayD), then the binary FP64
+// walk over those.
 cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const LaunchPlan &plan,
                          cudaStream_t stream, uint32_t *counters,
                          unsigned long long *totals = nullptr);

@@ -215,7 +215,9 @@ static void emu_pass(const bzr::SceneView &view, long n, const double *org, cons
                                  tmax ? tmax[i] : 1.7976931348623157e308);
       r.any_hit = (mode & 2) != 0;
       bzr::KState st;
-      if (mode & 1)
+      if (mode & 4)
+        bzr::traverse_mixed<KIND, false, bzr::RayD>(view.k[KIND], r, st, sk, 0, &e, nullptr);
+      else if (mode & 1)
         bzr::traverse_mixed<KIND, false>(view.k[KIND], r, st, sk, 0, &e, nullptr);
       else
         bzr::traverse<KIND, false>(view.k[KIND], r, st, sk, 0, &e, nullptr);

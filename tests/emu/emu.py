@@ -140,14 +140,15 @@ class EmuScene(_Base):
         return _closest_surface(self, points)
 
     def intersect(self, org, dirs, tmin=None, tmax=None, stack_cap=0, mode="fp64", any_hit=False):
-        """mode fp64 | mixed; any_hit: every ray with Ray::AnyHit::yes."""
+        """mode fp64 (the binary walk) | wide64 (the FP64 mode's wide walk) | mixed; any_hit: every
+        ray with Ray::AnyHit::yes."""
         org, dirs, tmin, tmax, n = _rays(org, dirs, tmin, tmax)
         out = _outputs(n)
         out["error_word"] = int(self._lib.emu_scene_intersect(
             self._h, n, _ptr(org, _dp), _ptr(dirs, _dp), _ptr(tmin, _dp), _ptr(tmax, _dp),
             _ptr(out["t"], _dp), _ptr(out["uv"], _dp), _ptr(out["normal"], _dp),
             _ptr(out["prim"], _u32p), _ptr(out["geom"], _u32p), _ptr(out["hit"], _u8p), stack_cap,
-            (1 if mode == "mixed" else 0) | (2 if any_hit else 0)))
+            {"fp64": 0, "mixed": 1, "wide64": 4}[mode] | (2 if any_hit else 0)))
         return out
 
     def work_counts(self, org, dirs, tmin=None, tmax=None, mode="fp64"):
