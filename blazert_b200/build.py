@@ -29,7 +29,8 @@ HOST_FLAGS = ["-std=c++17", "-O3", "-fPIC", "-ffp-contract=off", "-Wall", "-Wext
 CU_FLAGS = ARCH + ["-std=c++17", "-O3", "-lineinfo", "--fmad=false", "-Xcompiler",
                    "-fPIC,-ffp-contract=off", "-ccbin", CXX]
 
-SOURCES = [("scene.cpp", "cxx"), ("capi.cpp", "cxx"), ("trace.cu", "cu"), ("adjoint.cu", "cu"),
+SOURCES = [("scene.cpp", "cxx"), ("capi.cpp", "cxx"), ("trace.cu", "cu"), ("trace_small.cu", "cu"),
+           ("adjoint.cu", "cu"),
            ("noalloc.cu", "cu"), ("batch.cpp", "cxx"), ("gbuild.cu", "cu"), ("distance.cu", "cu"),
            ("scene_io.cpp", "cxx"), ("obj.cpp", "cxx")]
 HEADERS = ["layout.h", "scene.h", "trace.h", "trace_core.cuh", "adjoint.h", "capi_internal.h",

@@ -602,16 +602,12 @@ inline bool use_local(const SceneView &S, const LaunchPlan &plan) {
   return !plan.shared_stack && S.stack_cap <= kLocalStack;
 }
 
-// Whether a pass of KIND in `mode` over n rays walks the wide image (and defers the rays it
-// cannot).  The FP64 mode does with the thread-local stack, from kWide64MinRays rays on; its
-// counting kernels count the binary walk.  Below, the launch of the pass over the deferred rays
-// (2 to 3 us a kind) costs more than the walk saves: one ray on an icosphere 12.2 us binary,
-// 15.5 wide; 32 rays 44.3 and 40.4, and through three kinds 183 and 131 us.
-constexpr uint32_t kWide64MinRays = 32;
+// Whether a pass of KIND in `mode` walks the wide image (and hands on the rays it cannot).  The
+// FP64 mode does with the thread-local stack; its counting kernels count the binary walk.
 template <int KIND>
-bool walks_wide(const SceneView &S, int mode, const LaunchPlan &plan, bool count, uint32_t n) {
+bool walks_wide(const SceneView &S, int mode, const LaunchPlan &plan, bool count) {
   return KIND != kCylinders && S.k[KIND].present && S.k[KIND].n_prims && S.k[KIND].mixed_ok &&
-         (mode == kModeMixed || (use_local(S, plan) && !count && n >= kWide64MinRays));
+         (mode == kModeMixed || (use_local(S, plan) && !count));
 }
 
 using TraceFn = void (*)(SceneView, RayIO, int, uint32_t *, unsigned long long *);
@@ -652,7 +648,7 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
     return int(std::min<uint64_t>(uint64_t(blocks), (uint64_t(io.n) + th - 1) / th));
   };
   if constexpr (KIND != kCylinders) {
-    if (walks_wide<KIND>(S, mode, plan, COUNT, io.n)) {
+    if (walks_wide<KIND>(S, mode, plan, COUNT)) {
       const bool mixed = mode == kModeMixed;
       const TraceFn wide_fn = !mixed ? trace_wide64_kernel<KIND>
                               : local ? trace_kernel<KIND, false, true, true>()
@@ -756,6 +752,7 @@ cudaError_t trace_prepare(const SceneView &S, LaunchPlan *plan) {
   if ((e = prepare_kind<kMesh>(S, plan)) != cudaSuccess) return e;
   if ((e = prepare_kind<kSpheres>(S, plan)) != cudaSuccess) return e;
   if ((e = prepare_kind<kPlanes>(S, plan)) != cudaSuccess) return e;
+  if ((e = small_prepare(plan)) != cudaSuccess) return e;
   return prepare_kind<kCylinders>(S, plan);
 }
 
@@ -767,6 +764,7 @@ int trace_passes(const SceneView &S) {
 
 cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const LaunchPlan &plan,
                          cudaStream_t stream, uint32_t *counters, unsigned long long *totals) {
+  if (!totals && small_batch(S, plan, io.n)) return launch_small(S, io, plan, stream);
   cudaError_t e = cudaMemsetAsync(counters, 0, kTraceCounterWords * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
   RayIO sorted = io;

@@ -80,10 +80,26 @@ struct LaunchPlan {
   int blocks32[kNumKinds] = {0, 0, 0, 0};  // mixed-precision kernels
   int blocks64w[kNumKinds] = {0, 0, 0, 0};  // the FP64 mode's wide kernels
   int blocks_rest[kNumKinds] = {0, 0, 0, 0};  // the binary passes after wide ones
+  int small_blocks[kNumKinds] = {0, 0, 0, 0};  // resident blocks of the small kernel, by kinds
   RaySort sort;
   uint32_t sort_min_rays = 1u << 16;  // smaller batches are traced in their own order
   cudaMemPool_t pool = nullptr;       // stream-ordered scratch (keeps its memory mapped)
 };
+
+// Small batches (trace_small.cu): one launch for every kind.  done: for results in host memory,
+// how the kernel tells the host that all of them are there: once every block has counted itself
+// in *blocks (device, zero before and again after), the last one writes value, with the call's
+// error word (zero again after) in the upper half, to *flag (host memory).
+struct SmallDone {
+  uint32_t *blocks = nullptr;
+  unsigned long long *flag = nullptr;
+  uint32_t value = 0;
+};
+cudaError_t small_prepare(LaunchPlan *plan);
+// Whether a batch of n rays takes the small kernel.
+bool small_batch(const SceneView &S, const LaunchPlan &plan, uint32_t n);
+cudaError_t launch_small(const SceneView &S, const RayIO &io, const LaunchPlan &plan,
+                         cudaStream_t stream, const SmallDone &done = SmallDone());
 
 // Many scenes in one launch per kind (the batching form).  Rays of scene s occupy
 // [ray_offset[s], ray_offset[s+1]) of the concatenated arrays in io.  Chunks of at most
