@@ -307,7 +307,7 @@ static int commit_scene(bzr_scene *s, uint32_t flags, bool trees_given) {
       }
       if (!built) c.tree = bzr::build_tree(c.boxes, s->host.opt);
       depth = std::max(depth, c.tree.max_depth);
-      img[k] = bzr::flatten(s->host, k);
+      img[k] = bzr::flatten(s->host, k, 16, false);
     }
   } catch (const std::bad_alloc &) {
     return fail(BZR_ENOMEM, "host allocation failed during the build");
@@ -326,13 +326,14 @@ static int commit_scene(bzr_scene *s, uint32_t flags, bool trees_given) {
     total = align_up(total + std::max<size_t>(bytes, 1), 256);
     return off;
   };
-  size_t off_nodes64[4], off_wide[4], off_leaves[4], off_payload[4], off_ids[4], off_tri[4],
+  size_t off_nodes64[4], off_wide[4], off_box[4], off_payload[4], off_ids[4], off_tri[4],
       off_tv[4], off_pos[4], off_vnorm[4];
   uint32_t wide_stack = 0;
   for (int k = 0; k < bzr::kNumKinds; ++k) {
     off_nodes64[k] = place(img[k].nodes64.data(), img[k].nodes64.size() * sizeof(double));
     off_wide[k] = place(img[k].wide.data(), img[k].wide.size());
-    off_leaves[k] = place(img[k].leaves.data(), img[k].leaves.size() * sizeof(double));
+    // filled on the device from the nodes
+    off_box[k] = place(nullptr, img[k].mixed_ok ? img[k].prim_ids.size() * 6 * sizeof(double) : 0);
     if (img[k].mixed_ok) wide_stack = std::max(wide_stack, img[k].wide_stack);
     off_payload[k] = place(img[k].payload.data(), img[k].payload.size() * sizeof(double));
     off_ids[k] = place(img[k].prim_ids.data(), img[k].prim_ids.size() * sizeof(uint32_t));
@@ -364,7 +365,7 @@ static int commit_scene(bzr_scene *s, uint32_t flags, bool trees_given) {
   e = bzr::dev_malloc(&s->arena, total);
   if (e != cudaSuccess) return fail(BZR_ENOMEM, "device arena allocation failed");
   for (const Piece &p : pieces) {
-    if (!p.bytes) continue;
+    if (!p.bytes || !p.src) continue;
     e = cudaMemcpy(static_cast<char *>(s->arena) + p.off, p.src, p.bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "scene upload");
   }
@@ -377,9 +378,8 @@ static int commit_scene(bzr_scene *s, uint32_t flags, bool trees_given) {
     if (!c.present) continue;
     v.nodes64 = reinterpret_cast<const double *>(base + off_nodes64[k]);
     v.wide = reinterpret_cast<const unsigned char *>(base + off_wide[k]);
-    v.leaves = reinterpret_cast<const double *>(base + off_leaves[k]);
+    v.leaf_box = reinterpret_cast<const double *>(base + off_box[k]);
     v.n_wide = img[k].n_wide;
-    v.n_leaf16 = img[k].n_leaf16;
     v.wide_root_ref = img[k].wide_root_ref;
     v.payload = reinterpret_cast<const double *>(base + off_payload[k]);
     v.prim_ids = reinterpret_cast<const uint32_t *>(base + off_ids[k]);
@@ -394,6 +394,10 @@ static int commit_scene(bzr_scene *s, uint32_t flags, bool trees_given) {
     v.mixed_ok = img[k].mixed_ok ? 1 : 0;
     std::memcpy(v.root_box, img[k].root_box, sizeof v.root_box);
     v.coord_max = img[k].coord_max;
+    if (v.mixed_ok) {
+      e = bzr::fill_leaf_boxes(v, reinterpret_cast<double *>(base + off_box[k]));
+      if (e != cudaSuccess) return cuda_fail(e, "leaf boxes");
+    }
   }
   s->view.faces = reinterpret_cast<const uint32_t *>(base + off_faces);
   s->view.vert_n = reinterpret_cast<const double *>(base + off_vn);

@@ -57,17 +57,19 @@ constexpr int kVertexDoubles = 4;
 //   bytes 16..63  u8: for axis a, lo[8] at 16 + 16a and hi[8] at 24 + 16a; child c's box on
 //                 axis a is [origin + lo[c] * 2^e, origin + hi[c] * 2^e]; an unused slot has
 //                 lo = 255, hi = 0 (an empty box)
-//   bytes 64..95  u32 ref[8]: a wide node index, or kLeafBit | a leaf record's offset in
-//                 16-byte units
+//   bytes 64..95  u32 ref[8]: a wide node index, or kLeafBit | the leaf's first leaf-ordered
+//                 position, as in the binary nodes
 //   bytes 96..127 u32 perm[8]: for a ray of direction-sign octant s = sx | sy << 1 | sz << 2,
 //                 nibble j of perm[s] is the slot of the j-th child in the reference's visit
 //                 order, 15 past the last child (the reference visits
 //                 children[direction_sign[axis]] first at every binary node,
 //                 blazert/bvh/accel.h:100-104, so a treelet's order depends on s only).
-// Leaf records (16-byte aligned): the leaf's exact FP64 box (lo.x, hi.x, lo.y, hi.y, lo.z,
-// hi.z; 48 B), u32 first leaf-ordered position, u32 count, 8 B zero; then the leaf's
-// primitives: triangles {i0, i1, i2, 0} (16 B, indices into the vertex array), spheres and
-// planes their payload records (32 B, 112 B).
+// The leaves' exact FP64 boxes stand apart (KindView::leaf_box): a leaf's primitives are read
+// from the leaf-ordered arrays that the binary walk reads too, and its box only once one of them
+// is hit.  (The image can also be built with leaf records in place of these positions, refs then
+// being kLeafBit | the record's offset in 16-byte units: the box (lo.x, hi.x, lo.y, hi.y, lo.z,
+// hi.z; 48 B), u32 first leaf-ordered position, u32 count, 8 B zero; then the leaf's primitives,
+// triangles {i0, i1, i2, 0}, spheres and planes their payload records.)
 constexpr int kWideMax = 8;
 // Entries of the thread-local traversal stack; trees whose stack needs more (depth > 62,
 // reachable only with max_tree_depth above 62) trace with the stack in shared memory in FP64,
@@ -95,10 +97,10 @@ struct KindView {
   double root_box[6] = {0, 0, 0, 0, 0, 0};  // (lo.x, hi.x, lo.y, hi.y, lo.z, hi.z)
   // mixed-precision image (see kWideBytes); the root's wide node is index 0
   const unsigned char *wide = nullptr;   // n_wide * kWideBytes
-  const double *leaves = nullptr;        // leaf records, n_leaf16 16-byte units
+  const double *leaf_box = nullptr;      // 6 per leaf-ordered position: the box (lo.x, hi.x, ...)
+                                         // of the leaf that starts there
   uint32_t n_wide = 0;
-  uint32_t n_leaf16 = 0;
-  uint32_t wide_root_ref = 0;            // 0 (wide root) or kLeafBit | offset of a leaf root
+  uint32_t wide_root_ref = 0;            // 0 (wide root) or kLeafBit | position of a leaf root
   float coord_max = 0.0f;       // largest |coordinate| of the root box, rounded up
 };
 

@@ -548,13 +548,15 @@ bool axis_grid(double lo, double hi, int *e_out, int64_t *k_out) {
 // The mixed-precision image of one kind (layout.h, kWideBytes): leaf records in tree order,
 // then the wide nodes breadth-first from the root's treelet.  Leaves the image's mixed_ok
 // false when a box cannot be quantised or the traversal stack could exceed kLocalStack.
-void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, KindImage *img) {
+void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, bool records,
+                KindImage *img) {
   const size_t nn = t.nodes.size();
   const uint32_t units = kind == kMesh ? 1u : uint32_t(kPayloadDoubles[kind] * 8 / 16);
   // leaf records: 4 units of header, then `units` per primitive
-  std::vector<uint32_t> leaf_off(nn, 0);
+  std::vector<uint32_t> leaf_off(records ? nn : 0, 0);
+  auto leaf_ref = [&](uint32_t x) { return kLeafBit | (records ? leaf_off[x] : leaf_pos[x]); };
   uint64_t total = 0;
-  for (size_t i = 0; i < nn; ++i)
+  for (size_t i = 0; records && i < nn; ++i)
     if (t.nodes[i].leaf == 1) {
       leaf_off[i] = static_cast<uint32_t>(total);
       total += kLeafHeaderBytes / 16 + uint64_t(units) * t.nodes[i].prim_cnt;
@@ -564,7 +566,7 @@ void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, 
     return;
   }
   img->leaves.resize(size_t(total) * 2);
-  for (size_t i = 0; i < nn; ++i) {
+  for (size_t i = 0; records && i < nn; ++i) {
     const TreeNode &nd = t.nodes[i];
     if (nd.leaf != 1) continue;
     double *L = &img->leaves[size_t(leaf_off[i]) * 2];
@@ -590,7 +592,7 @@ void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, 
   img->n_wide = 0;
   img->wide_stack = 1;
   if (t.nodes[0].leaf == 1) {
-    img->wide_root_ref = kLeafBit | leaf_off[0];
+    img->wide_root_ref = leaf_ref(0);
     return;
   }
   img->wide_root_ref = 0;
@@ -661,7 +663,7 @@ void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, 
     for (size_t j = 0; j < ch.size(); ++j) {
       const TreeNode &c = t.nodes[ch[j]];
       if (c.leaf == 1) {
-        ref[j] = kLeafBit | leaf_off[ch[j]];
+        ref[j] = leaf_ref(ch[j]);
       } else {
         ref[j] = static_cast<uint32_t>(queue.size());
         queue.push_back(ch[j]);
@@ -701,7 +703,7 @@ void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, 
   img->wide_coord_max = round_up(cmax);
 }
 
-KindImage flatten(const HostScene &s, int kind, size_t max_workers) {
+KindImage flatten(const HostScene &s, int kind, size_t max_workers, bool records) {
   const Collection &c = s.kind[kind];
   const Tree &t = c.tree;
   KindImage img;
@@ -821,7 +823,7 @@ KindImage flatten(const HostScene &s, int kind, size_t max_workers) {
     number_vertices(s, &img, range_workers(np, kPrimsPerRange, max_workers));
   // Cylinders may move the hit distance outward (blazert/primitives/cylinder.h:181-495), which
   // the wide image's exactness argument excludes; their mixed mode runs the FP64 traversal.
-  if (img.mixed_ok && kind != kCylinders && nn) build_wide(t, kind, leaf_pos, &img);
+  if (img.mixed_ok && kind != kCylinders && nn) build_wide(t, kind, leaf_pos, records, &img);
   else img.mixed_ok = false;
   return img;
 }

@@ -170,12 +170,15 @@ struct KindImage {
   bool mixed_ok = true;         // the wide image was built
 };
 
-// Builds the mixed-precision image of a flattened kind (called by flatten).
-void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, KindImage *img);
+// Builds the wide image of a flattened kind (called by flatten).
+void build_wide(const Tree &t, int kind, const std::vector<uint32_t> &leaf_pos, bool records,
+                KindImage *img);
 
 // Device image of one kind's tree and primitives.  Long loops run on up to max_workers threads;
-// the image does not depend on how many.
-KindImage flatten(const HostScene &s, int kind, size_t max_workers = 16);
+// the image does not depend on how many.  records: the wide nodes refer to leaf records (which
+// hold each leaf's box and primitives: a self-contained image, used to check it); without them
+// they refer to the leaf's first leaf-ordered position, which is what the kernels walk.
+KindImage flatten(const HostScene &s, int kind, size_t max_workers = 16, bool records = true);
 
 // Persistent scene format (scene_io.cpp): a committed scene's inputs, build options and trees
 // as bytes, and back.  decode_scene fills a fresh HostScene (primitives added, trees checked

@@ -96,13 +96,10 @@ __device__ __forceinline__ void prefetch_l2(const void *base, size_t bytes) {
 
 template <int KIND, bool WIDE>
 __device__ __forceinline__ void prefetch_kind(const KindView &K) {
-  if (WIDE && K.mixed_ok) {  // the wide image: nodes, then leaf records (and vertices)
+  if (WIDE && K.mixed_ok)
     prefetch_l2(K.wide, size_t(K.n_wide) * kWideBytes);
-    prefetch_l2(K.leaves, size_t(K.n_leaf16) * 16);
-    if (KIND == kMesh) prefetch_l2(K.verts, size_t(K.n_verts) * kVertexDoubles * sizeof(double));
-    return;
-  }
-  prefetch_l2(K.nodes64, size_t(K.n_internal) * kNode64Doubles * sizeof(double));
+  else
+    prefetch_l2(K.nodes64, size_t(K.n_internal) * kNode64Doubles * sizeof(double));
   if (KIND == kMesh) {
     prefetch_l2(K.tri, size_t(K.n_prims) * 4 * sizeof(uint32_t));
     prefetch_l2(K.verts, size_t(K.n_verts) * kVertexDoubles * sizeof(double));
@@ -595,6 +592,19 @@ __global__ void sort_histogram_kernel(RayIO io, RaySort rs, uint32_t *keys, uint
   }
 }
 
+__global__ void leaf_box_kernel(KindView K, double *leaf_box) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < K.n_internal;
+       i += gridDim.x * blockDim.x) {
+    const double *nd = K.nodes64 + size_t(i) * kNode64Doubles;
+    const uint32_t *ref = reinterpret_cast<const uint32_t *>(nd + 12);
+    for (int c = 0; c < 2; ++c) {
+      if (!(ref[c] & kLeafBit) || (ref[c] & kIdMask) >= K.n_prims) continue;
+      double *out = leaf_box + size_t(ref[c] & kIdMask) * 6;
+      for (int j = 0; j < 6; ++j) out[j] = nd[6 * c + j];
+    }
+  }
+}
+
 // The counting kernels (measurement only) always keep the stack in shared memory; the
 // tracing kernels use the thread-local stack whenever the tree's stack fits it, unless the
 // plan asks for shared memory.
@@ -731,6 +741,15 @@ cudaError_t launch_defaults(const RayIO &io, int sms, cudaStream_t stream) {
   const int blocks = int(want < uint64_t(sms) * 8 ? (want ? want : 1) : uint64_t(sms) * 8);
   fill_defaults_kernel<<<blocks, threads, 0, stream>>>(io);
   return cudaGetLastError();
+}
+
+cudaError_t fill_leaf_boxes(const KindView &K, double *leaf_box) {
+  if (K.root_ref & kLeafBit)
+    return cudaMemcpy(leaf_box, K.root_box, sizeof K.root_box, cudaMemcpyHostToDevice);
+  const uint32_t blocks = (K.n_internal + 255) / 256;
+  leaf_box_kernel<<<blocks < 1184 ? blocks : 1184, 256>>>(K, leaf_box);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
 }
 
 size_t trace_smem_bytes(uint32_t stack_cap, int threads) {

@@ -154,6 +154,9 @@ cudaError_t launch_batch(const BatchView &B, const RayIO &io, int mode, const Ba
 // RayHit defaults for every ray of io (a scene without primitives).
 cudaError_t launch_defaults(const RayIO &io, int sms, cudaStream_t stream);
 
+// Fills K's leaf_box (device, 6 doubles per primitive position) from its nodes and root box.
+cudaError_t fill_leaf_boxes(const KindView &K, double *leaf_box);
+
 size_t trace_smem_bytes(uint32_t stack_cap, int threads);
 // Dynamic shared memory of a trace_kind_kernel launch: the stack unless thread-local, then
 // top_nodes staged 128-byte nodes.

@@ -1128,58 +1128,69 @@ BZR_HD void wtrav_to_leaf(const KindView &K, const Ray &r, const F &f, typename 
   if (tv.post == kNoLeaf && !tv.walk) tv.live = false;  // nothing left to process
 }
 
-// The first postponed leaf record: the exact FP64 test of the leaf's box, then its primitives in
-// the reference's stored order (blazert/bvh/intersect.h:67-78); the queue moves up by one.  The
-// walk then resumes at tv.cur.
+// The first postponed leaf: its primitives in the reference's stored order
+// (blazert/bvh/intersect.h:67-78); the queue moves up by one.  The walk then resumes at tv.cur.
+//
+// The reference tests the leaf's own box first (intersect.h:33-51) and skips the leaf when that
+// fails.  The box decides nothing unless a primitive of the leaf is hit, so it is read and tested
+// only then, against the hit distance from before the leaf, and a failed test takes the leaf's
+// hits back.  Most leaves are left without a hit: their boxes are never read, and without them
+// a leaf is just its primitives in the leaf-ordered arrays (16 bytes per triangle, where records
+// with their boxes took 112 for three triangles).
+// B200, FP64 mode: 8.4M bounce rays on a 2M-triangle terrain 4,610 -> 4,422 us (DRAM reads of a
+// 2M-ray launch 1.96 -> 1.19 GB), 1M shadow rays 636 -> 610, 1M rays through spheres, cylinders
+// and planes 1,385 -> 1,374; mixed mode unchanged.
 template <int KIND, bool COUNT, class F>
 BZR_HD void wtrav_leaf(const KindView &K, const Ray &r, const F &f, KState &st,
                        typename F::Bound &hl, Trav &tv, uint32_t *err, Counts *cnt) {
-  constexpr uint32_t kUnits = KIND == kMesh ? 1u : uint32_t(kPayloadDoubles[KIND] / 2);
   if (tv.post == kNoLeaf) return;
-  const uint32_t off = tv.post & kIdMask;
+  const uint32_t first = tv.post & kIdMask;
   tv.post = tv.post2;
   tv.post2 = kNoLeaf;
-  if (uint64_t(off) + kLeafHeaderBytes / 16 > K.n_leaf16) {
-    flag_error(err, kErrPrimIndex);
-    tv.live = false;
-    return;
-  }
-  const double *L = K.leaves + 2 * size_t(off);
-  const double2 px = ld2(L), py = ld2(L + 2), pz = ld2(L + 4);
-  const uint4 hdr = ldg(reinterpret_cast<const uint4 *>(L + 6));
+  const KState before = st;
+  auto box_passes = [&] {
+    const double *b = K.leaf_box + 6 * size_t(first);
+    double key;
+    return box_test(ld2(b), ld2(b + 2), ld2(b + 4), r, key) && !(key > before.hit);
+  };
+  // the counting kernels test it first, as the reference does, so that they count its tests
   if (COUNT) cnt->leaf[KIND] += 1;
-  double key;
-  if (box_test(px, py, pz, r, key) && !(key > st.hit)) {
-    if (uint64_t(off) + kLeafHeaderBytes / 16 + uint64_t(kUnits) * hdr.y > K.n_leaf16 ||
-        uint64_t(hdr.x) + hdr.y > K.n_prims) {
-      flag_error(err, kErrPrimIndex);
-      tv.live = false;
-      return;
-    }
-    const double before = st.hit;
-    for (uint32_t j = 0; j < hdr.y; ++j) {
-      const uint32_t pos = hdr.x + j;
-      const double *P = L + kLeafHeaderBytes / 8 + size_t(j) * kUnits * 2;
+  if (!COUNT || box_passes()) {
+    bool any = false;
+    for (uint32_t pos = first;; ++pos) {
+      if (pos >= K.n_prims) {
+        flag_error(err, kErrPrimIndex);
+        tv.live = false;
+        return;
+      }
       if (COUNT) cnt->prim[KIND] += 1;
       bool h;
-      if (KIND == kMesh)
-        h = isect_triangle<false>(K.verts, ldg(reinterpret_cast<const uint4 *>(P)), pos, r, st);
-      else if (KIND == kSpheres)
-        h = isect_sphere(P, pos, r, st);
-      else
-        h = isect_plane(P, pos, r, st);
-      if (h && r.any_hit) {  // the first hit ends the leaf and the traversal
-        tv.live = false;
-        return;
+      uint32_t id;
+      if (KIND == kMesh) {
+        const uint4 w = ldg(reinterpret_cast<const uint4 *>(K.tri) + pos);
+        id = w.w;
+        h = isect_triangle<false>(K.verts, w, pos, r, st);
+      } else {
+        id = isect<KIND>(K, pos, r, st, h);
       }
+      any |= h;
+      if ((id & kLastBit) || (h && r.any_hit)) break;
     }
-    if (st.hit != before) {
-      if (!(st.hit < before)) {  // moved outward, or NaN (see RayD)
-        tv.post = kRedoLeaf;
-        tv.live = false;
-        return;
+    if (any) {
+      if (!COUNT && !box_passes()) {
+        st = before;
+      } else {
+        if (r.any_hit) {  // the first hit ends the leaf and the traversal
+          tv.live = false;
+          return;
+        }
+        if (!(st.hit <= before.hit)) {  // moved outward, or NaN (see RayD)
+          tv.post = kRedoLeaf;
+          tv.live = false;
+          return;
+        }
+        hl = hit_bound(f, st.hit);
       }
-      hl = hit_bound(f, st.hit);
     }
   }
   if (!tv.walk && tv.post == kNoLeaf) tv.live = false;

@@ -15,7 +15,9 @@
 namespace {
 struct Emu {
   bzr::HostScene host;
-  std::vector<bzr::KindImage> img;
+  std::vector<bzr::KindImage> img;              // with leaf records (emu_wide_check)
+  std::vector<bzr::KindImage> dev;              // as the product uploads it
+  std::vector<std::vector<double>> leaf_box;    // as fill_leaf_boxes fills it
   bzr::SceneView view;
 };
 }  // namespace
@@ -24,6 +26,8 @@ struct Emu {
 static void commit(Emu *e, bool build) {
   bzr::HostScene &s = e->host;
   e->img.resize(4);
+  e->dev.resize(4);
+  e->leaf_box.resize(4);
   uint32_t depth = 0;
   for (int k = 0; k < 4; ++k) {
     bzr::Collection &c = s.kind[k];
@@ -34,12 +38,24 @@ static void commit(Emu *e, bool build) {
     if (build) c.tree = bzr::build_tree(c.boxes, s.opt);
     depth = depth > c.tree.max_depth ? depth : c.tree.max_depth;
     e->img[k] = bzr::flatten(s, k);
-    const bzr::KindImage &im = e->img[k];
+    e->dev[k] = bzr::flatten(s, k, 16, false);
+    const bzr::KindImage &im = e->dev[k];
+    std::vector<double> &box = e->leaf_box[k];
+    box.assign(im.prim_ids.size() * 6, 0.0);
+    auto leaf_box = [&](uint32_t ref, const double *b) {
+      if (ref & bzr::kLeafBit) std::memcpy(&box[6 * size_t(ref & bzr::kIdMask)], b, 48);
+    };
+    if (!box.empty()) leaf_box(im.root_ref, im.root_box);
+    for (uint32_t g = 0; g < im.n_internal; ++g) {
+      const double *nd = &im.nodes64[size_t(g) * bzr::kNode64Doubles];
+      uint32_t ref[2];
+      std::memcpy(ref, nd + 12, sizeof ref);
+      for (int c = 0; c < 2; ++c) leaf_box(ref[c], nd + 6 * c);
+    }
     v.nodes64 = im.nodes64.data();
     v.wide = im.wide.data();
-    v.leaves = im.leaves.data();
+    v.leaf_box = box.data();
     v.n_wide = im.n_wide;
-    v.n_leaf16 = im.n_leaf16;
     v.wide_root_ref = im.wide_root_ref;
     v.payload = im.payload.data();
     v.prim_ids = im.prim_ids.data();
