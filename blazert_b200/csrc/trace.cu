@@ -366,11 +366,13 @@ constexpr auto trace_kernel() {
 // keeps its own ray's scene, so a warp may finish rays of one scene while starting another's.
 // The pass of a scene's first kind writes its whole record; the pass of its last kind
 // completes it and stamps the scene's completion time.
-// LCAP: entries of the thread-local stack (the batch's stack-depth knob: 32 or 64).
-template <int KIND, bool MIXED, bool LOCAL, uint32_t LCAP>
+// LCAP: entries of the thread-local stack (the batch's stack-depth knob: 32 or 64).  F: the walk,
+// as in trace_kind_body; rays that a wide walk does not cover take the binary one in the same
+// kernel.
+template <int KIND, class F, bool LOCAL, uint32_t LCAP>
 __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO &io,
                                                  uint32_t *chunk_counter, uint32_t stack_cap) {
-  constexpr bool kWide = MIXED && KIND != kCylinders;
+  constexpr bool kWide = !std::is_same<F, NoWalk>::value && KIND != kCylinders;
   extern __shared__ __align__(16) unsigned char smem[];
   double lkey[LOCAL ? LCAP : 1];
   uint32_t lref[LOCAL ? LCAP : 1];
@@ -385,9 +387,9 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
   uint32_t i = 0, sc = 0;
   const KindView *K = nullptr;
   Ray r;
-  RayW f;
-  float hl = 0.0f;
-  bool use32 = false;
+  F f;
+  typename F::Bound hl = 0;
+  bool wide = false;
   KState st;
   Trav tv;
   Counts cnt = {};
@@ -439,13 +441,17 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
                        io.tmax ? io.tmax[i] : kDblMax);
           r.any_hit = io.any_hit != 0;
           if constexpr (kWide) {
-            f = make_ray_f(r, static_cast<const RayW *>(nullptr));
-            use32 = K->mixed_ok && f.ok;
+            f = make_ray_f(r, static_cast<const F *>(nullptr));
+            wide = K->mixed_ok && f.ok;
           }
-          if (kWide && use32)
-            wtrav_begin<KIND, false>(*K, r, f, st, hl, tv, &cnt);
-          else
-            trav_begin<KIND, false>(*K, r, st, tv, &cnt);
+          bool begun = false;
+          if constexpr (kWide) {
+            if (wide) {
+              wtrav_begin<KIND, false>(*K, r, f, st, hl, tv, &cnt);
+              begun = true;
+            }
+          }
+          if (!begun) trav_begin<KIND, false>(*K, r, st, tv, &cnt);
         }
       }
       if (want > avail) {
@@ -463,24 +469,45 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
     }
     if (!__any_sync(kFull, active)) break;
     if (active) {
-      if (kWide && use32) {
-        if (tv.live) wtrav_to_leaf<KIND, false>(*K, r, f, hl, tv, sk, tid, io.error_word, &cnt);
-        while (tv.live && tv.post != kNoLeaf)
-          wtrav_leaf<KIND, false>(*K, r, f, st, hl, tv, io.error_word, &cnt);
-        if (!tv.live && tv.post == kRedoLeaf) {  // rare: the binary walk, from the start
-          use32 = false;
-          trav_begin<KIND, false>(*K, r, st, tv, &cnt);
+      bool stepped = false;
+      if constexpr (kWide) {
+        if (wide) {
+          if (tv.live) wtrav_to_leaf<KIND, false>(*K, r, f, hl, tv, sk, tid, io.error_word, &cnt);
+          // as in trace_kind_body: what only the leaf steps read is formed again here
+          r.tmin = io.tmin ? ldg(io.tmin + i) : 0.0;
+          r.any_hit = io.any_hit != 0;
+          r.sx = f.oct & 1u, r.sy = (f.oct >> 1) & 1u, r.sz = f.oct >> 2;
+          while (tv.live && tv.post != kNoLeaf)
+            wtrav_leaf<KIND, false>(*K, r, f, st, hl, tv, io.error_word, &cnt);
+          if (!tv.live && tv.post == kRedoLeaf) {  // rare: the binary walk, from the start
+            wide = false;
+            r.tmax = io.tmax ? ldg(io.tmax + i) : kDblMax;
+            trav_begin<KIND, false>(*K, r, st, tv, &cnt);
+          }
+          stepped = true;
         }
-      } else {
+      }
+      if (!stepped) {
         if (tv.live) trav_to_leaf<KIND, false>(*K, r, st, tv, sk, tid, io.error_word, &cnt);
         if (tv.live) trav_leaf<KIND, false>(*K, r, st, tv, sk, tid, io.error_word, &cnt);
       }
       if (!tv.live) {
-        if (kWide && use32) wtrav_end<KIND>(*K, r, st);
+        if constexpr (kWide) {
+          r.tmax = io.tmax ? ldg(io.tmax + i) : kDblMax;
+          if (wide) wtrav_end<KIND>(*K, r, st);
+        }
         finalize_kind<KIND>(B.views[sc], r, st, i, B.first_kind[sc] == KIND, io.t, io.uv,
                             io.normal, io.prim, io.geom, io.hit);
-        if (B.last_kind[sc] == KIND && B.scene_left) {
-          if (atomicSub(B.scene_left + sc, 1u) == 1u && B.scene_done_ns) {
+        // The count of a scene's unfinished rays serves the completion stamps only.  Most rays
+        // in flight belong to one or two scenes, and an atomic per ray on their counters set the
+        // pace of the whole batch (3M rays in 48 scenes, mixed:
+        // 2,140 -> 1,514 us without them): without stamps nothing is counted, and with
+        // them the lanes that finish together count once per scene.
+        if (B.scene_done_ns && B.last_kind[sc] == KIND) {
+          const unsigned same = __match_any_sync(__activemask(), sc);
+          const uint32_t done = __popc(same);
+          if (lane == unsigned(__ffs(same)) - 1u &&
+              atomicSub(B.scene_left + sc, done) == done) {
             __threadfence();
             unsigned long long now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -493,26 +520,37 @@ __device__ __forceinline__ void trace_batch_body(const BatchView &B, const RayIO
   }
 }
 
-// The batch's FP64 kernels, and its mixed kernels under a register cap, as trace_wide_kernel.
-// The batch's scenes are small and mostly in L2, so its walk waits less on memory: on 256
-// icospheres the cap measured 1,180 (none), 1,188 (72), 1,224 (80) and 1,215 (96) Mrays/s.
-#ifndef BZR_BATCH_WIDE_REGS
-#define BZR_BATCH_WIDE_REGS 80
-#endif
+// The batch's binary kernels, and its wide kernels under a register cap, as trace_wide_kernel.
+// 3M rays in 48 icosphere scenes, mixed mode: 72 / 80 / 88 / 96 registers 1,560 / 1,514 / 1,621 /
+// 1,599 us.
+constexpr int kBatchWideRegs = 80;
 template <int KIND, bool LOCAL, uint32_t LCAP>
 __global__ void __launch_bounds__(kMaxTraceThreads)
     trace_batch_kernel(BatchView B, RayIO io, uint32_t *chunk_counter, uint32_t stack_cap) {
-  trace_batch_body<KIND, false, LOCAL, LCAP>(B, io, chunk_counter, stack_cap);
+  trace_batch_body<KIND, NoWalk, LOCAL, LCAP>(B, io, chunk_counter, stack_cap);
 }
 template <int KIND, bool LOCAL, uint32_t LCAP>
-__global__ void __maxnreg__(BZR_BATCH_WIDE_REGS)
+__global__ void __maxnreg__(kBatchWideRegs)
     trace_batch_wide_kernel(BatchView B, RayIO io, uint32_t *chunk_counter, uint32_t stack_cap) {
-  trace_batch_body<KIND, true, LOCAL, LCAP>(B, io, chunk_counter, stack_cap);
+  trace_batch_body<KIND, RayW, LOCAL, LCAP>(B, io, chunk_counter, stack_cap);
 }
-template <int KIND, bool MIXED, bool LOCAL, uint32_t LCAP>
+// FP64 mode, 3M rays in 48 icosphere scenes: the binary walk 2,163 us, the wide one with 80 /
+// 88 / 96 / 112 registers 1,598 / 1,658 / 1,615 / 1,796 us.
+constexpr int kBatchWide64Regs = 80;
+template <int KIND, uint32_t LCAP>
+__global__ void __maxnreg__(kBatchWide64Regs)
+    trace_batch_wide64_kernel(BatchView B, RayIO io, uint32_t *chunk_counter, uint32_t stack_cap) {
+  trace_batch_body<KIND, RayD, true, LCAP>(B, io, chunk_counter, stack_cap);
+}
+// The walk of a batch's pass: the binary one (cylinders; the FP64 mode with the stack in shared
+// memory; node width 2), or the wide one in FP32 or FP64.
+enum BatchWalk { kBinary, kWide32, kWide64 };
+template <int KIND, int WALK, bool LOCAL, uint32_t LCAP>
 constexpr auto batch_fn() {
-  if constexpr (MIXED)
+  if constexpr (WALK == kWide32)
     return trace_batch_wide_kernel<KIND, LOCAL, LCAP>;
+  else if constexpr (WALK == kWide64 && LOCAL && KIND != kCylinders)
+    return trace_batch_wide64_kernel<KIND, LCAP>;
   else
     return trace_batch_kernel<KIND, LOCAL, LCAP>;
 }
@@ -859,27 +897,37 @@ cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const La
 namespace {
 // The kernel a batch launch uses for one kind: stack storage (thread-local with 32 or 64
 // entries, or shared) and mode.
-template <int KIND, bool MIXED>
-const void *batch_kernel(bool local, uint32_t lcap) {
-  if (local && lcap == 32) return reinterpret_cast<const void *>(batch_fn<KIND, MIXED, true, 32>());
-  if (local) return reinterpret_cast<const void *>(batch_fn<KIND, MIXED, true, kLocalStack>());
-  return reinterpret_cast<const void *>(batch_fn<KIND, MIXED, false, kLocalStack>());
+using BatchFn = void (*)(BatchView, RayIO, uint32_t *, uint32_t);
+template <int KIND, int WALK>
+BatchFn batch_kernel(bool local, uint32_t lcap) {
+  if (local && lcap == 32) return batch_fn<KIND, WALK, true, 32>();
+  if (local) return batch_fn<KIND, WALK, true, kLocalStack>();
+  return batch_fn<KIND, WALK, false, kLocalStack>();
 }
 
 inline bool batch_local(uint32_t stack_cap, const BatchPlan &plan) {
   return !plan.shared_stack && stack_cap <= plan.local_stack;
 }
 
+// The kernel of one kind's pass in `mode`.
 template <int KIND>
-cudaError_t prepare_batch_kind(uint32_t stack_cap, const BatchPlan &plan, int *blocks,
-                               int *blocks32) {
-  const int sms = plan.sms, th = plan.threads;
-  const bool local = batch_local(stack_cap, plan);
-  const size_t smem = local ? 0 : trace_smem_bytes(stack_cap, th);
-  const cudaError_t e = grid_for(batch_kernel<KIND, false>(local, plan.local_stack), th, smem, sms,
-                                 blocks);
+BatchFn batch_pass(int mode, const BatchPlan &plan) {
+  const bool local = batch_local(plan.stack_cap, plan);
+  if (KIND == kCylinders || (mode == kModeMixed && plan.node_width != 8))
+    return batch_kernel<KIND, kBinary>(local, plan.local_stack);
+  if (mode == kModeMixed) return batch_kernel<KIND, kWide32>(local, plan.local_stack);
+  return batch_kernel<KIND, kWide64>(local, plan.local_stack);
+}
+
+template <int KIND>
+cudaError_t prepare_batch_kind(const BatchPlan &plan, int *blocks, int *blocks32) {
+  const size_t smem = batch_local(plan.stack_cap, plan)
+                          ? 0 : trace_smem_bytes(plan.stack_cap, plan.threads);
+  const cudaError_t e = grid_for(reinterpret_cast<const void *>(batch_pass<KIND>(kModeFp64, plan)),
+                                 plan.threads, smem, plan.sms, blocks);
   if (e != cudaSuccess) return e;
-  return grid_for(batch_kernel<KIND, true>(local, plan.local_stack), th, smem, sms, blocks32);
+  return grid_for(reinterpret_cast<const void *>(batch_pass<KIND>(kModeMixed, plan)), plan.threads,
+                  smem, plan.sms, blocks32);
 }
 }  // namespace
 
@@ -891,16 +939,16 @@ cudaError_t batch_prepare(uint32_t stack_cap, BatchPlan *plan) {
   if (e != cudaSuccess) return e;
   plan->sms = sms;
   plan->stack_cap = stack_cap;
-  if ((e = prepare_batch_kind<kMesh>(stack_cap, *plan, &plan->blocks[kMesh],
-                                     &plan->blocks32[kMesh])) != cudaSuccess)
+  if ((e = prepare_batch_kind<kMesh>(*plan, &plan->blocks[kMesh], &plan->blocks32[kMesh])) !=
+      cudaSuccess)
     return e;
-  if ((e = prepare_batch_kind<kSpheres>(stack_cap, *plan, &plan->blocks[kSpheres],
+  if ((e = prepare_batch_kind<kSpheres>(*plan, &plan->blocks[kSpheres],
                                         &plan->blocks32[kSpheres])) != cudaSuccess)
     return e;
-  if ((e = prepare_batch_kind<kPlanes>(stack_cap, *plan, &plan->blocks[kPlanes],
+  if ((e = prepare_batch_kind<kPlanes>(*plan, &plan->blocks[kPlanes],
                                        &plan->blocks32[kPlanes])) != cudaSuccess)
     return e;
-  return prepare_batch_kind<kCylinders>(stack_cap, *plan, &plan->blocks[kCylinders],
+  return prepare_batch_kind<kCylinders>(*plan, &plan->blocks[kCylinders],
                                         &plan->blocks32[kCylinders]);
 }
 
@@ -927,41 +975,16 @@ cudaError_t launch_batch(const BatchView &B, const RayIO &io, int mode, const Ba
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     run.perm = sort_scratch.perm;
   }
-  const bool local = batch_local(plan.stack_cap, plan);
-  const int th = plan.threads;
-  const size_t smem = local ? 0 : trace_smem_bytes(plan.stack_cap, th);
+  const size_t smem = batch_local(plan.stack_cap, plan)
+                          ? 0 : trace_smem_bytes(plan.stack_cap, plan.threads);
   for (int k = 0; k < kNumKinds; ++k) {
     if (!(plan.kinds_present & (1 << k))) continue;
-    // cylinders, and every kind at node width 2: the FP64 traversal
-    const bool m = mode == kModeMixed && k != kCylinders && plan.node_width == 8;
-    const int b = m ? plan.blocks32[k] : plan.blocks[k];
-    uint32_t *c = counters + k;
-#define BZR_BATCH_LAUNCH(KK)                                                                   \
-  if (local && plan.local_stack == 32) {                                                       \
-    if (m)                                                                                     \
-      batch_fn<KK, true, true, 32>()<<<b, th, 0, stream>>>(B, run, c, plan.stack_cap);          \
-    else                                                                                       \
-      batch_fn<KK, false, true, 32>()<<<b, th, 0, stream>>>(B, run, c, plan.stack_cap);         \
-  } else if (local) {                                                                          \
-    if (m)                                                                                     \
-      batch_fn<KK, true, true, kLocalStack>()<<<b, th, 0, stream>>>(B, run, c, plan.stack_cap); \
-    else                                                                                       \
-      batch_fn<KK, false, true, kLocalStack>()<<<b, th, 0, stream>>>(B, run, c,                 \
-                                                                   plan.stack_cap);            \
-  } else if (m) {                                                                              \
-    batch_fn<KK, true, false, kLocalStack>()<<<b, th, smem, stream>>>(B, run, c,                \
-                                                                    plan.stack_cap);           \
-  } else {                                                                                     \
-    batch_fn<KK, false, false, kLocalStack>()<<<b, th, smem, stream>>>(B, run, c,               \
-                                                                     plan.stack_cap);          \
-  }
-    switch (k) {
-      case kMesh: BZR_BATCH_LAUNCH(kMesh); break;
-      case kSpheres: BZR_BATCH_LAUNCH(kSpheres); break;
-      case kPlanes: BZR_BATCH_LAUNCH(kPlanes); break;
-      default: BZR_BATCH_LAUNCH(kCylinders); break;
-    }
-#undef BZR_BATCH_LAUNCH
+    const BatchFn fn = k == kMesh      ? batch_pass<kMesh>(mode, plan)
+                       : k == kSpheres ? batch_pass<kSpheres>(mode, plan)
+                       : k == kPlanes  ? batch_pass<kPlanes>(mode, plan)
+                                       : batch_pass<kCylinders>(mode, plan);
+    const int blocks = mode == kModeMixed ? plan.blocks32[k] : plan.blocks[k];
+    fn<<<blocks, plan.threads, smem, stream>>>(B, run, counters + k, plan.stack_cap);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -265,7 +265,7 @@ int bzr_scene_check(const bzr_scene *scene, void *stream, int timeout_ms, uint32
 /* Node width of a batch's walk in BZR_MODE_MIXED (batches only, bzr_batch_tune): 8 (the
  * default) walks the 8-wide nodes with the FP32 child tests, 2 the binary FP64 nodes of the FP64
  * mode.  Both process the same leaves in the same order, so the results are the same bits;
- * BZR_MODE_FP64 always walks the binary nodes. */
+ * BZR_MODE_FP64 walks the wide nodes with FP64 tests at either setting. */
 #define BZR_TUNE_NODE_WIDTH 12
 int bzr_scene_tune(bzr_scene *scene, int option, int64_t value);
 
