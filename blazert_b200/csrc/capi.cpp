@@ -549,9 +549,13 @@ static int run_small(bzr_scene *s, size_t n, const double *org, const double *di
   // the block for kSmallBatch rays with every piece bounds what any small batch needs
   const size_t cap = 8 * align_up(24 * kSmallBatch, 256) + 512;
   const bool direct = !totals && bzr::small_batch(s->view, s->plan, static_cast<uint32_t>(n));
-  if (!s->small_pin && bzr::host_malloc(&s->small_pin, cap) != cudaSuccess) {
-    s->small_pin = nullptr;
-    return fail(BZR_ENOMEM, "pinned staging allocation failed");
+  if (!s->small_pin) {
+    if (bzr::host_malloc(&s->small_pin, cap) != cudaSuccess) {
+      s->small_pin = nullptr;
+      return fail(BZR_ENOMEM, "pinned staging allocation failed");
+    }
+    // the flag of another scene's block may lie where this one's is: no call has this value
+    std::memset(s->small_pin + cap - 256, 0, 256);
   }
   if (!direct && s->stage_bytes < cap) {
     cudaFree(s->stage_dev);
@@ -586,7 +590,8 @@ static int run_small(bzr_scene *s, size_t n, const double *org, const double *di
     bzr::SmallDone done;
     done.blocks = s->slots + kSmallWords;
     done.flag = flag;
-    done.value = ++s->small_calls;
+    if (++s->small_calls == 0) ++s->small_calls;  // 0: no call yet
+    done.value = s->small_calls;
     const cudaError_t e = bzr::launch_small(s->view, ci, s->plan, st, done);
     if (e != cudaSuccess) return cuda_fail(e, "small batch submission");
     // spin for as long as such a batch may take, then the bounded wait for the stream, which

@@ -90,3 +90,23 @@ def test_small_batches_on_many_streams():
     assert bad == []
     assert scene.check() == 0
     scene.close()
+
+
+def test_a_new_scene_does_not_see_an_earlier_scenes_flag():
+    """The flag that ends a small host-array call lies in pinned memory that a closed scene may
+    have used for its own: the first calls of a new scene wait for their own results."""
+    import blazert_b200 as B
+
+    rng = np.random.default_rng(4)
+    for k in range(12):
+        c, r = rng.uniform(-1.0, 1.0, (50, 3)), rng.uniform(0.1, 0.4, 50)
+        spec = W.SceneSpec().add_spheres(c, r)
+        scene, ora = product_scene(spec), Oracle(spec)
+        for _ in range(3):
+            o = 4.0 * W._unit_sphere(rng, 1)
+            d = rng.uniform(-0.5, 0.5, (1, 3)) - o
+            ref = ora.intersect(o, d)
+            hit, rh = scene.intersect1(B.Ray(o[0], d[0]))
+            assert hit == bool(ref["hit"][0]) and rh.prim_id == ref["prim"][0], k
+            assert not hit or rh.hit_distance == ref["t"][0]
+        scene.close()
