@@ -136,6 +136,115 @@ struct Rest {
   using Bound = float;
 };
 
+// The first kernel of a wide pass: each warp looks through its share of the batch for rays that
+// the wide walk leaves out and traces them through the binary nodes, lanes refilled as they
+// finish; the wide kernel runs beside it.  These rays start first because they can be the
+// slowest: the middle row of an image of odd height has a zero direction component, and along a
+// plane of box bounds the reference's 0 * inf accepts thousands of boxes.  Traced after the wide
+// kernel instead, they added their whole time to it: 541,501 pixels of a 20,480-triangle sphere
+// 637 us, now 396; without that row 166.  (As a first phase, or a last one, inside the wide
+// kernel they cost the walk its registers: 8.4M bounce rays on a terrain 4,420 -> 4,560 to 4,850
+// us; a look through those takes about 10.)
+constexpr uint32_t kScan = 8;  // runs of 32 rays a warp looks at together: independent loads
+template <int KIND, bool COUNT, class F, bool LOCAL>
+__global__ void __launch_bounds__(kMaxTraceThreads)
+    trace_left_out_kernel(SceneView S, RayIO io, int first, uint32_t *,
+                          unsigned long long *totals) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const KindView &K = S.k[KIND];
+  double lkey[LOCAL ? kLocalStack : 1];
+  uint32_t lref[LOCAL ? kLocalStack : 1];
+  Stack sk;
+  uint32_t tid;
+  init_stack<LOCAL>(sk, tid, S.stack_cap, smem, lkey, lref);
+  if (!COUNT) prefetch_kind<KIND, true>(K);
+  Counts cnt = {};
+  // The wide kernel starts once every block is here, with whatever preceded this pass complete.
+  griddep_wait();
+  griddep_launch_dependents();
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  // runs of 32 rays, dealt to the warps in turn (left-out rays tend to lie together), kScan runs
+  // looked at together
+  uint64_t run = warp;
+  const uint64_t runs = (uint64_t(io.n) + 31) / 32;
+  unsigned found[kScan] = {};  // warp-uniform: the left-out rays of the runs, not yet taken
+  uint64_t at = 0;             // the first of these runs
+  uint32_t i = 0;
+  bool active = false;
+  Ray r;
+  KState st;
+  Trav tv;
+  auto any_found = [&] {
+    unsigned m = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kScan; ++j) m |= found[j];
+    return m != 0;
+  };
+  for (;;) {
+    const unsigned idle = __ballot_sync(kFull, !active);
+    while (idle && run < runs && !any_found()) {
+#pragma unroll
+      for (uint32_t j = 0; j < kScan; ++j) {
+        const uint64_t idx = (run + uint64_t(j) * warps) * 32 + lane;
+        bool out = false;
+        if (idx < io.n) {
+          const double w[3] = {io.dir[3 * idx], io.dir[3 * idx + 1], io.dir[3 * idx + 2]};
+          out = left_out(w, io.tmin ? io.tmin[idx] : 0.0, io.tmax ? io.tmax[idx] : kDblMax,
+                         static_cast<const F *>(nullptr));
+        }
+        found[j] = __ballot_sync(kFull, out);
+      }
+      at = run;
+      run += uint64_t(kScan) * warps;
+    }
+    if (idle && any_found()) {  // the idle lanes take found rays in their order
+      uint32_t rank = __popc(idle & below), left = __popc(idle);
+      bool got = false;
+#pragma unroll
+      for (uint32_t j = 0; j < kScan; ++j) {
+        const uint32_t have = __popc(found[j]);
+        if (!active && !got && rank < have) {
+          unsigned m = found[j];
+          for (uint32_t k = 0; k < rank; ++k) m &= m - 1;
+          i = uint32_t((at + uint64_t(j) * warps) * 32) + unsigned(__ffs(m)) - 1u;
+          got = true;
+        }
+        if (!got) rank -= have < rank ? have : rank;
+        const uint32_t taken = left < have ? left : have;
+        for (uint32_t k = 0; k < taken; ++k) found[j] &= found[j] - 1;
+        left -= taken;
+      }
+      if (got) {
+        active = true;
+        r = make_ray(io.org + 3 * size_t(i), io.dir + 3 * size_t(i), io.tmin ? io.tmin[i] : 0.0,
+                     io.tmax ? io.tmax[i] : kDblMax);
+        r.any_hit = io.any_hit != 0;
+        trav_begin<KIND, COUNT>(K, r, st, tv, &cnt);
+      }
+    }
+    if (!__any_sync(kFull, active)) {
+      if (run >= runs && !any_found()) break;
+      continue;
+    }
+    if (active) {
+      if (tv.live) trav_to_leaf<KIND, COUNT>(K, r, st, tv, sk, tid, io.error_word, &cnt);
+      if (tv.live) trav_leaf<KIND, COUNT>(K, r, st, tv, sk, tid, io.error_word, &cnt);
+      if (!tv.live) {
+        finalize_kind<KIND>(S, r, st, i, first != 0, io.t, io.uv, io.normal, io.prim, io.geom,
+                            io.hit);
+        active = false;
+      }
+    }
+  }
+  if (COUNT) {
+    unsigned long long v[4] = {cnt.box[KIND], cnt.prim[KIND], cnt.node[KIND], cnt.leaf[KIND]};
+    for (int j = 0; j < 4; ++j)
+      if (v[j]) atomicAdd(totals + j * kNumKinds + KIND, v[j]);
+  }
+}
+
 template <int KIND, bool COUNT, class F, bool LOCAL>
 __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO &io, int first,
                                                 uint32_t *work_counter,
@@ -168,8 +277,9 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
     sk.n_top = n_top;
   }
   // Up to here only the scene was read; the counters, the rays' closest distances and the
-  // lists come from earlier kernels of the stream.
-  griddep_wait();
+  // lists come from earlier kernels of the stream.  (What precedes a wide kernel's first kernel
+  // is complete, and these two trace different rays; see the end.)
+  if constexpr (!kWide) griddep_wait();
   // The rays of a Rest pass: the listed ones, or every ray that the wide walk does not cover
   // when they outgrew their list, or every ray when those to redo outgrew theirs (a ray the
   // wide walk has finished gives the same result again).
@@ -200,6 +310,7 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
     for (;;) {  // refill the idle lanes; repeats only after a lane handed its ray on
       const unsigned idle = __ballot_sync(kFull, !active);
       bool deferred = false;
+      bool skipped = false;
       if (idle && !exhausted) {
         const uint32_t want = __popc(idle), avail = pool_end - pool_next;
         // rays taken per fetch: io.chunk (>= 32, so one fetch serves every idle lane), or
@@ -229,20 +340,25 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
             r.any_hit = io.any_hit != 0;
             if constexpr (kWide) {
               f = make_ray_f(r, static_cast<const F *>(nullptr));
-              if (K.mixed_ok && f.ok) {
+              if (f.ok) {
                 wtrav_begin<KIND, COUNT>(K, r, f, st, hl, tv, &cnt);
-              } else {
+              } else {  // the pass's first kernel has it, or it is handed on
                 active = false;
-                deferred = true;
+                skipped = true;
+                deferred = !left_out(io.dir + 3 * size_t(i), r.tmin, r.tmax,
+                                     static_cast<const F *>(nullptr));
               }
             } else {
-              if constexpr (kRest) {  // the wide walk has traced the rays it covers
+              if constexpr (kRest) {  // the wide pass has traced the others
+                const double *w = io.dir + 3 * size_t(i);
                 if (scan && !all && idx < io.n &&
                     (io.wide_mode == kModeMixed
-                         ? make_ray_f(r, static_cast<const RayW *>(nullptr)).ok
-                         : make_ray_f(r, static_cast<const RayD *>(nullptr)).ok)) {
+                         ? left_out(w, r.tmin, r.tmax, static_cast<const RayW *>(nullptr)) ||
+                               make_ray_f(r, static_cast<const RayW *>(nullptr)).ok
+                         : left_out(w, r.tmin, r.tmax, static_cast<const RayD *>(nullptr)) ||
+                               make_ray_f(r, static_cast<const RayD *>(nullptr)).ok)) {
                   active = false;
-                  deferred = true;
+                  skipped = true;
                 }
               }
               if (active) trav_begin<KIND, COUNT>(K, r, st, tv, &cnt);
@@ -258,10 +374,10 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
         }
       }
       if constexpr (!kWide && !kRest) break;
-      const unsigned handed = __ballot_sync(kFull, deferred);
-      if (!handed) break;
+      if (!__any_sync(kFull, skipped)) break;
       if constexpr (kWide) {
-        if (!list_full) {
+        const unsigned handed = __ballot_sync(kFull, deferred);
+        if (handed && !list_full) {
           uint32_t at = 0;
           if (lane == 0) at = atomicAdd(io.uncovered_count, __popc(handed));
           at = __shfl_sync(kFull, at, 0);
@@ -303,6 +419,7 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
       }
     }
   }
+  if constexpr (kWide) griddep_wait();  // this grid is not complete before the pass's first one
   if (COUNT) {
     for (int k = 0; k < kNumKinds; ++k) {
       unsigned long long v[4] = {cnt.box[k], cnt.prim[k], cnt.node[k], cnt.leaf[k]};
@@ -342,7 +459,7 @@ constexpr int kWide64Regs = 80;
 template <int KIND>
 __global__ void __maxnreg__(kWide64Regs)
     trace_wide64_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
-                        unsigned long long *totals) {
+                      unsigned long long *totals) {
   trace_kind_body<KIND, false, RayD, true>(S, io, first, work_counter, totals);
 }
 
@@ -650,12 +767,20 @@ inline bool use_local(const SceneView &S, const LaunchPlan &plan) {
   return !plan.shared_stack && S.stack_cap <= kLocalStack;
 }
 
-// Whether a pass of KIND in `mode` walks the wide image (and hands on the rays it cannot).  The
-// FP64 mode does with the thread-local stack; its counting kernels count the binary walk.
+// Whether a pass of KIND in `mode` walks the wide image.  The FP64 mode does with the thread-local
+// stack; its counting kernels count the binary walk.
+//
+// A mesh of less than kWideMinTriangles triangles keeps the binary walk: its nodes lie in L1 and
+// a binary step is then the cheaper one.  543,004 / 91,204 pixels of a 320-triangle sphere 66 /
+// 39 us binary, 76 / 48 wide; of a 1,280-triangle one 100 / 66 and 98 / 62.  (500 spheres and 100
+// planes gain by the wide walk: 1M rays through spheres, planes and cylinders 1,380 against
+// 1,359, a fitting step with 500 spheres 1,450 against 1,413.)
+constexpr uint32_t kWideMinTriangles = 512;
 template <int KIND>
 bool walks_wide(const SceneView &S, int mode, const LaunchPlan &plan, bool count) {
   return KIND != kCylinders && S.k[KIND].present && S.k[KIND].n_prims && S.k[KIND].mixed_ok &&
-         (mode == kModeMixed || (use_local(S, plan) && !count));
+         (mode == kModeMixed || (use_local(S, plan) && !count &&
+                                 (KIND != kMesh || S.k[KIND].n_prims >= kWideMinTriangles)));
 }
 
 using TraceFn = void (*)(SceneView, RayIO, int, uint32_t *, unsigned long long *);
@@ -709,11 +834,19 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
       wide.uncovered = counters + kTraceListWord;
       wide.redo = wide.uncovered + kUncoveredList;
       wide.wide_mode = mode;
-      const cudaError_t e =
-          launch_one(wide_fn, grid(mixed ? plan.blocks32[KIND] : plan.blocks64w[KIND]), th, smem,
-                     stream, early, S, wide, first, counters + KIND, totals);
+      const TraceFn out_fn =
+          mixed ? (local ? trace_left_out_kernel<KIND, false, RayW, true>
+                         : trace_left_out_kernel<KIND, COUNT, RayW, false>)
+                : trace_left_out_kernel<KIND, false, RayD, true>;
+      cudaError_t e = launch_one(out_fn, grid(plan.blocks_out[KIND]), th, smem, stream, early, S,
+                                 wide, first, nullptr, totals);
       if (e != cudaSuccess) return e;
-      return launch_one(rest_fn, grid(plan.blocks_rest[KIND]), th, smem, stream,
+      e =
+          launch_one(wide_fn, grid(mixed ? plan.blocks32[KIND] : plan.blocks64w[KIND]), th,
+                     smem, stream, plan.early_launch, S, wide, first, counters + KIND, totals);
+      if (e != cudaSuccess) return e;
+      // hardly ever any ray: a small grid, which leaves the SMs to the next pass
+      return launch_one(rest_fn, grid(std::min(plan.blocks_rest[KIND], plan.sms)), th, smem, stream,
                         plan.early_launch, S, wide, first, counters + kNumKinds + KIND, totals);
     }
   }
@@ -761,12 +894,20 @@ cudaError_t prepare_kind(const SceneView &S, LaunchPlan *plan) {
                                reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, false>)};
     for (const void *fn : rest_fns)
       if (e == cudaSuccess) e = grid_for(fn, th, smem, plan->sms, &plan->blocks_rest[KIND]);
+    const void *out_fns[4] = {
+        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, true, RayW, false>),
+        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayW, false>),
+        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayW, true>),
+        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayD, true>)};
+    for (int j = 0; j < (local ? 4 : 2); ++j)
+      if (e == cudaSuccess)
+        e = grid_for(out_fns[j], th, j < 2 ? smem : bytes, plan->sms, &plan->blocks_out[KIND]);
     if (local && e == cudaSuccess)
       e = grid_for(reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, true>), th, bytes,
                    plan->sms, &plan->blocks_rest[KIND]);
     if (local && e == cudaSuccess)
-      e = grid_for(reinterpret_cast<const void *>(trace_wide64_kernel<KIND>), th, bytes, plan->sms,
-                   &plan->blocks64w[KIND]);
+      e = grid_for(reinterpret_cast<const void *>(trace_wide64_kernel<KIND>), th,
+                   bytes, plan->sms, &plan->blocks64w[KIND]);
   }
   return e;
 }
@@ -798,6 +939,7 @@ size_t trace_kind_smem(uint32_t stack_cap, int threads, bool local, uint32_t top
   const size_t stack = local ? 0 : (trace_smem_bytes(stack_cap, threads) + 15) / 16 * 16;
   return stack + size_t(top_nodes) * 128;
 }
+
 
 cudaError_t trace_prepare(const SceneView &S, LaunchPlan *plan) {
   int dev = 0, sms = 0;

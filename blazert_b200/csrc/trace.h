@@ -45,11 +45,11 @@ struct RayIO {
   uint32_t chunk = kRayChunk;      // rays a warp takes per fetch: 32, 64, 128, or 0 for
                                    // exactly the lanes that are idle
   uint32_t top_nodes = 0;          // top-level nodes each block stages in shared memory
-  // Wide passes: the rays the wide walk does not cover, or whose walk ends without a result,
-  // are counted here and the first of each noted in the lists, for the binary pass right after.
-  // A batch has few such rays or (axis-parallel ones) many: a short list that needs no
-  // allocation serves the few, and past it the binary pass looks at every ray again.  Set by
-  // launch_trace.
+  // Wide passes: the rays that the pass's first kernel leaves to the walk but that the walk does
+  // not cover (origins beyond its range), or whose walk ends without a result, are counted here
+  // and the first of each noted in the lists, for the binary pass right after.  A batch has
+  // hardly any: a short list needs no allocation, and past it the binary pass looks at every ray
+  // again.  Set by launch_trace.
   uint32_t *uncovered_count = nullptr, *redo_count = nullptr;
   uint32_t *uncovered = nullptr, *redo = nullptr;
   int wide_mode = 0;  // the mode whose wide pass handed the rays on (its cover test)
@@ -79,6 +79,7 @@ struct LaunchPlan {
   int blocks[kNumKinds] = {0, 0, 0, 0};    // FP64 kernels
   int blocks32[kNumKinds] = {0, 0, 0, 0};  // mixed-precision kernels
   int blocks64w[kNumKinds] = {0, 0, 0, 0};  // the FP64 mode's wide kernels
+  int blocks_out[kNumKinds] = {0, 0, 0, 0};   // the first kernels of wide passes
   int blocks_rest[kNumKinds] = {0, 0, 0, 0};  // the binary passes after wide ones
   int small_blocks[kNumKinds] = {0, 0, 0, 0};  // resident blocks of the small kernel, by kinds
   RaySort sort;
@@ -172,10 +173,10 @@ int trace_passes(const SceneView &S);
 // counters: kTraceWords device words, zeroed here as far as needed.  totals (device, 8 x uint64,
 // or null): when given, the counting kernels add per kind the box tests (totals[0..3]) and
 // primitive tests (totals[4..7]) of every ray.
-// A pass of a kind whose wide image exists is two kernels: the wide walk over the batch, which
-// hands on the rays it does not cover (FP32: a direction component of 0 or below 2^-40 in
-// magnitude, an origin coordinate or tmin beyond 1e18, NaN; FP64: RayD), then the binary FP64
-// walk over those.
+// A pass of a kind whose wide image exists is three kernels: the binary walk of the rays that the
+// wide walk leaves out (FP32: a direction component of 0 or below 2^-40 in magnitude, a tmin
+// beyond 1e18, NaN; FP64: RayD), beside it the wide walk of the others, then the binary walk of
+// those that the wide walk hands on.
 cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const LaunchPlan &plan,
                          cudaStream_t stream, uint32_t *counters,
                          unsigned long long *totals = nullptr);

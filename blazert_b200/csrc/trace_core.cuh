@@ -709,6 +709,29 @@ BZR_HD float f32_down(double x) {  // x rounded toward -inf
 #endif
 }
 
+// Whether a wide walk with FP32 (RayW) or FP64 (RayD) tests leaves a ray out for its direction or
+// its range: exactly the conditions of make_ray_f's ok but for the origin's, with the divisions
+// only near their bounds (1 / w is rounded once).
+BZR_HD int32_t hi_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double2hiint(x);
+#else
+  return static_cast<int32_t>(dbits(x) >> 32);
+#endif
+}
+// 2^lo <= |x| < 2^hi, on the high word (false for 0, NaN and infinities)
+BZR_HD bool in_range(double x, int lo, int hi) {
+  const uint32_t e = uint32_t(hi_word(x)) & 0x7FFFFFFFu;
+  return e - (uint32_t(1023 + lo) << 20) < (uint32_t(hi - lo) << 20);
+}
+BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayW *) {
+  bool in = in_range(w[0], -39, 1000) && in_range(w[1], -39, 1000) && in_range(w[2], -39, 1000);
+  if (!in) {
+    in = true;
+    for (int a = 0; a < 3; ++a) in = in && fabs(1.0 / w[a]) > 0.0 && fabs(1.0 / w[a]) <= 0x1p40;
+  }
+  return !(in && fabs(tmin) <= 1e18 && !isnan(tmax));
+}
 BZR_HD RayW make_ray_f(const Ray &r, const RayW *) {
   RayW f;
   const double inv[3] = {r.inv.x, r.inv.y, r.inv.z}, o[3] = {r.o.x, r.o.y, r.o.z};
@@ -776,13 +799,6 @@ struct RayD {
   bool ok;
 };
 
-BZR_HD int32_t hi_word(double x) {
-#if defined(__CUDA_ARCH__)
-  return __double2hiint(x);
-#else
-  return static_cast<int32_t>(dbits(x) >> 32);
-#endif
-}
 BZR_HD double from_hi(uint32_t hi) {  // the double with this high word and a zero low word
 #if defined(__CUDA_ARCH__)
   return __hiloint2double(static_cast<int>(hi), 0);
@@ -821,6 +837,15 @@ BZR_HD float hit_bound(const RayW &, double h) {
 }
 BZR_HD int32_t hit_bound(const RayD &, double h) { return h == 0.0 ? 0 : hi_word(h); }
 
+BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayD *) {
+  bool in = in_range(w[0], -499, 499) && in_range(w[1], -499, 499) && in_range(w[2], -499, 499);
+  if (!in) {
+    in = true;
+    for (int a = 0; a < 3; ++a)
+      in = in && fabs(1.0 / w[a]) >= 0x1p-500 && fabs(1.0 / w[a]) <= 0x1p500;
+  }
+  return !(in && tmin >= 0.0 && !isnan(tmax));
+}
 BZR_HD RayD make_ray_f(const Ray &r, const RayD *) {
   RayD f;
   const double inv[3] = {r.inv.x, r.inv.y, r.inv.z}, o[3] = {r.o.x, r.o.y, r.o.z};

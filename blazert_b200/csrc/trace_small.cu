@@ -53,38 +53,34 @@ __device__ __forceinline__ void trace_lanes(const SceneView &S, const Ray &r, bo
                                             const Stack &sk, uint32_t *err, KState &st) {
   const KindView &K = S.k[KIND];
   constexpr bool kWide = KIND != kCylinders;
-  RayD f;
-  int32_t hl = 0;
   Trav tv;
-  bool active = mine, wide = false;
-  if (active) {
-    if constexpr (kWide) {
-      f = make_ray_f(r, static_cast<const RayD *>(nullptr));
-      wide = K.mixed_ok && f.ok;
-    }
-    if (kWide && wide)
-      wtrav_begin<KIND, false>(K, r, f, st, hl, tv, nullptr);
-    else
-      trav_begin<KIND, false>(K, r, st, tv, nullptr);
-  }
-  while (__any_sync(kFull, active)) {
-    if (active) {
-      if (kWide && wide) {
+  bool binary = mine;
+  if constexpr (kWide) {
+    const RayD f = make_ray_f(r, static_cast<const RayD *>(nullptr));
+    bool active = mine && K.mixed_ok && f.ok;
+    binary = mine && !active;
+    int32_t hl = 0;
+    if (active) wtrav_begin<KIND, false>(K, r, f, st, hl, tv, nullptr);
+    while (__any_sync(kFull, active)) {
+      if (active) {
         if (tv.live) wtrav_to_leaf<KIND, false>(K, r, f, hl, tv, sk, 0, err, nullptr);
         while (tv.live && tv.post != kNoLeaf)
           wtrav_leaf<KIND, false>(K, r, f, st, hl, tv, err, nullptr);
-        if (!tv.live && tv.post == kRedoLeaf) {  // rare: the binary walk, from the start
-          wide = false;
-          trav_begin<KIND, false>(K, r, st, tv, nullptr);
+        if (!tv.live) {
+          active = false;
+          binary = tv.post == kRedoLeaf;  // rare: the binary walk, from the start
+          if (!binary) wtrav_end<KIND>(K, r, st);
         }
-      } else {
-        if (tv.live) trav_to_leaf<KIND, false>(K, r, st, tv, sk, 0, err, nullptr);
-        if (tv.live) trav_leaf<KIND, false>(K, r, st, tv, sk, 0, err, nullptr);
       }
-      if (!tv.live) {
-        if (kWide && wide) wtrav_end<KIND>(K, r, st);
-        active = false;
-      }
+    }
+  }
+  // A loop of its own: rays along a plane of box bounds take thousands of its steps.
+  if (binary) trav_begin<KIND, false>(K, r, st, tv, nullptr);
+  while (__any_sync(kFull, binary)) {
+    if (binary) {
+      if (tv.live) trav_to_leaf<KIND, false>(K, r, st, tv, sk, 0, err, nullptr);
+      if (tv.live) trav_leaf<KIND, false>(K, r, st, tv, sk, 0, err, nullptr);
+      binary = tv.live;
     }
   }
 }
@@ -104,7 +100,7 @@ __device__ __forceinline__ void write_result(const SceneView &S, const RayIO &io
 __global__ void __maxnreg__(kRegs)
     trace_small_kernel(SceneView S, RayIO io, const SmallArgs args) {
   __shared__ double rays[32 * 8];  // origin, direction, tmin, tmax of each lane's ray
-  __shared__ Partial part[kNumKinds][32];
+  extern __shared__ Partial part[];  // the kinds' results, 32 each; none for a single kind
   double lkey[kLocalStack];
   uint32_t lref[kLocalStack];
   Stack sk;
@@ -142,22 +138,25 @@ __global__ void __maxnreg__(kRegs)
     case kPlanes: trace_lanes<kPlanes>(S, r, mine, sk, io.error_word, st); break;
     default: trace_lanes<kCylinders>(S, r, mine, sk, io.error_word, st); break;
   }
-  part[warp][lane] = Partial{st.hit, st.u, st.v, st.n.x, st.n.y, st.n.z, st.pos};
-  __syncthreads();
+  const Partial own = {st.hit, st.u, st.v, st.n.x, st.n.y, st.n.z, st.pos};
+  if (args.n_kinds > 1) {
+    part[32 * warp + lane] = own;
+    __syncthreads();
+  }
   // The merge of finalize_kind over the kinds in their order: a kind's hit replaces what was
   // there when it is strictly closer (triangles come first and always do).
   if (warp == 0 && mine) {
     int win = 0;
     double best = kDblMax;
-    for (int k = 0; k < args.n_kinds; ++k) {
-      const double h = part[k][lane].hit;
+    for (int k = 0; args.n_kinds > 1 && k < args.n_kinds; ++k) {
+      const double h = part[32 * k + lane].hit;
       if (h < r.tmax && (args.kind[k] == kMesh || h < best)) {
         win = k;
         best = h;
       }
     }
     // without a hit, the first kind's record (a miss) writes the defaults
-    const Partial &p = part[win][lane];
+    const Partial p = args.n_kinds > 1 ? part[32 * win + lane] : own;
     const uint64_t i = uint64_t(first) + lane;
     switch (args.kind[win]) {
       case kMesh: write_result<kMesh>(S, io, r, p, i); break;
@@ -186,26 +185,32 @@ __global__ void __maxnreg__(kRegs)
 
 }  // namespace
 
+// Shared memory is L1 that the walks lack: a single kind's blocks take none for the merge.
+static size_t small_smem(int kinds) { return kinds > 1 ? size_t(kinds) * 32 * sizeof(Partial) : 0; }
+
 cudaError_t small_prepare(LaunchPlan *plan) {
   for (int k = 1; k <= kNumKinds; ++k) {
     int per_sm = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, reinterpret_cast<const void *>(trace_small_kernel), 32 * k, 0);
+        &per_sm, reinterpret_cast<const void *>(trace_small_kernel), 32 * k, small_smem(k));
     if (e != cudaSuccess) return e;
     plan->small_blocks[k - 1] = plan->sms * std::max(1, per_sm);
   }
   return cudaSuccess;
 }
 
-// The line lies where the batch no longer fits the GPU in one wave of full warps: 32 rays a block,
-// as many blocks as are resident with a warp per kind.  B200, this kernel against the persistent
-// ones: three kinds (23,680 rays) 97 / 172 us at 16,384, 131 / 176 at 24,000, 276 / 207 at
-// 65,536; one kind (75,776 rays) 52 / 63 at 16,384, 61 / 72 at 65,536.
+// The line lies where the batch no longer fits the GPU in one wave: as many blocks as are resident
+// with a warp per kind, of 32 rays, or of 8 with a single kind.  B200, this kernel against the
+// persistent ones: three kinds (23,680 rays) 97 / 172 us at 16,384, 131 / 176 at 24,000, 276 / 207
+// at 65,536.  One kind (18,944 rays): 16,384 pixels of a 20,480-triangle sphere 69 / 102; up to
+// 75,776 rays it would still gain on most images (68,510 pixels 62 / 82), but where a row of
+// rays runs along a plane of box bounds (an odd number of rows) the persistent kernels' first
+// pass is the faster one: 67,405 pixels 660 / 399, 32,761 pixels 718 / 573.
 bool small_batch(const SceneView &S, const LaunchPlan &plan, uint32_t n) {
   const int kinds = trace_passes(S);
   return kinds > 0 && !plan.shared_stack && S.stack_cap <= kLocalStack &&
          !(plan.sort.enabled && n >= plan.sort_min_rays) &&
-         n <= 32u * uint32_t(plan.small_blocks[kinds - 1]);
+         n <= (kinds > 1 ? 32u : 8u) * uint32_t(plan.small_blocks[kinds - 1]);
 }
 
 cudaError_t launch_small(const SceneView &S, const RayIO &io, const LaunchPlan &plan,
@@ -216,7 +221,8 @@ cudaError_t launch_small(const SceneView &S, const RayIO &io, const LaunchPlan &
   const uint32_t blocks = uint32_t(plan.small_blocks[a.n_kinds - 1]);
   a.lanes = std::min<uint32_t>(32u, (io.n + blocks - 1) / blocks);
   a.done = done;
-  trace_small_kernel<<<(io.n + a.lanes - 1) / a.lanes, 32 * a.n_kinds, 0, stream>>>(S, io, a);
+  trace_small_kernel<<<(io.n + a.lanes - 1) / a.lanes, 32 * a.n_kinds, small_smem(a.n_kinds),
+                       stream>>>(S, io, a);
   return cudaGetLastError();
 }
 
