@@ -19,8 +19,8 @@ directions), float64, seeded.  A step is one intersectN over the whole batch.
              arrays): host->device copy of the rays, the kernel, device->host copy of all
              results, every step.
   roofline   the FP64 traversal kernel against two measured ceilings: algorithmic bytes (ray
-             I/O 121 B + 64 B per box test + the primitive record per primitive test; counts
-             from the counting kernel) against the L2 read bandwidth measured in the run
+             I/O 121 B + 128 B per wide node (cylinders 64 B per box test) + the primitive
+             record per primitive test; counts from the counting kernel) against the L2 read bandwidth measured in the run
              (bound "l2"), and the compulsory bytes (ray I/O + the scene's device image once)
              against the HBM copy bandwidth (MEASURED_PEAKS.json).
   cpu_baseline  the reference's own intersect1 loop (its headers, release flags, OpenMP over
@@ -550,17 +550,18 @@ def run_ours(args):
             "step_ms_min_max": [min(res["mixed"]["step_ms"]), max(res["mixed"]["step_ms"])]}
     # one traversal kernel per primitive kind present, per step
     n_passes = sum(1 for k in wl.scene.order if len(next(iter(getattr(wl.scene, k).values()))))
-    # kernels per call: one per kind present; in the mixed mode the triangle, sphere and plane
-    # passes add the FP64 pass over the rays their FP32 test does not cover
+    # kernels per call: one per kind present; the triangle, sphere and plane passes add one before
+    # the wide walk, for the rays it leaves out, and one after it, for those it hands on
     n_wide = sum(1 for k in wl.scene.order
                  if k != "cylinders" and len(next(iter(getattr(wl.scene, k).values()))))
-    launches_per_call = {"fp64": n_passes, "mixed": n_passes + n_wide}
+    launches_per_call = {"fp64": n_passes + 2 * n_wide, "mixed": n_passes + 2 * n_wide}
 
-    # roofline of the primary path's traversal kernel.  Algorithmic bytes from the kernel's own
-    # work counts (untimed counting run): ray I/O + 64 B per box test (half a 128-byte two-child
-    # node) + the primitive record per primitive test.
-    counts = scene.work_counts(o, d, tmn, tmx, stream=stream)
-    alg_bytes = n * RAY_IO_BYTES + BOX_TEST_BYTES * sum(counts["box"]) + \
+    # roofline of the primary path's traversal kernels.  Algorithmic bytes from the walk's own work
+    # counts (untimed counting run): ray I/O + 128 B per wide node (cylinders: 64 B per box test,
+    # half a 128-byte two-child node) + the primitive record per primitive test.
+    counts = scene.work_counts(o, d, tmn, tmx, stream=stream, mode="mixed")
+    alg_bytes = n * RAY_IO_BYTES + 128 * sum(counts["node"][:3]) + \
+        BOX_TEST_BYTES * counts["box"][3] + \
         sum(PRIM_RECORD_BYTES[k] * counts["prim"][k] for k in range(4))
     mean_ms = statistics.mean(step_ms)
     achieved = alg_bytes / (mean_ms / 1e3) / 1e9
@@ -823,7 +824,8 @@ def run_adjoint(args):
                        "l2": "flushed between timed steps (256 MiB write)"},
             "adjoint_ms_per_step": adj_ms / args.steps, "hit_fraction": hit_frac,
             "e2e": e2e,
-            "gpu_launches": args.steps * 4,  # two kind passes, the ray and face adjoint kernels
+            # two kind passes of three kernels, the ray and face adjoint kernels
+            "gpu_launches": args.steps * 8,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "peak_source": peak_src},
             "cpu_baseline": cpu, "clocks": clocks}), flush=True)

@@ -220,7 +220,9 @@ int bzr_work_counts(const bzr_scene *scene, size_t n, const double *origins,
  * the box tests (FP64: as above; mixed: the root test plus every child of every wide node
  * fetched), in totals[4..7] the primitive tests, in totals[8..11] the node fetches (FP64
  * internal nodes, or wide nodes) and in totals[12..15] the leaf fetches (FP64: leaves whose
- * primitives run; mixed: leaf records read, each with its exact FP64 box test). */
+ * primitives run; mixed: leaves reached, each with its exact FP64 box test).  The FP64 counts
+ * are the reference's own tests, those of the binary walk; the tracing kernels of either mode
+ * walk the wide nodes. */
 int bzr_work_counts_ex(const bzr_scene *scene, size_t n, const double *origins,
                        const double *directions, const double *tmin, const double *tmax,
                        int mode, uint64_t totals[16], void *stream);
@@ -244,7 +246,8 @@ int bzr_scene_check(const bzr_scene *scene, void *stream, int timeout_ms, uint32
 #define BZR_TUNE_BLOCK 3
 #define BZR_TUNE_STACK 4
 #define BZR_TUNE_CHUNK 5
-/* Host-array calls: the batch is split into at most this many chunks (1 to 32, default 8) of
+/* Host-array calls from pinned memory (and of less than 196,608 rays from ordinary memory): the
+ * batch is split into at most this many chunks (1 to 32, default 8) of
  * at least BZR_TUNE_HOST_MIN_CHUNK rays (default 131,072), pipelined as copies in, kernels and
  * copies out. */
 #define BZR_TUNE_HOST_CHUNKS 6
