@@ -4,7 +4,8 @@
 // order (triangles, spheres, planes, cylinders; blazert/scene.h:161-210).  Each pass merges its
 // hits into the output record with the reference's rule (finalize_kind), so the result equals
 // intersect1's.  Splitting by kind keeps each kernel small (registers, instruction cache) and
-// keeps one kind's nodes and primitives hot in L1/L2 at a time.
+// keeps one kind's nodes and primitives hot in L1/L2 at a time.  (Batches that fit the GPU in one
+// wave take the one launch of trace_small.cu instead.)
 //
 // Work distribution: each warp owns a pool of ray indices taken from a global counter in
 // chunks of kChunk (one atomic per chunk).  A lane whose ray finishes takes the next index of
@@ -803,9 +804,10 @@ cudaError_t launch_one(TraceFn fn, int blocks, int threads, size_t smem, cudaStr
   return cudaLaunchKernelEx(&cfg, fn, S, io, first, counter, totals);
 }
 
-// The pass of one kind: one kernel, or for a wide walk the wide kernel and then the FP64
-// kernel over the rays it deferred.  counters: the kTraceCounterWords words of the call;
-// after_trace: a trace kernel of this call precedes the pass on the stream.
+// The pass of one kind: one kernel, or for a wide walk three: the binary walk of the rays it leaves
+// out, beside it the wide kernel, then the binary walk of the rays that one handed on.  counters:
+// the kTraceWords words of the call; after_trace: a trace kernel of this call precedes the pass on
+// the stream.
 template <int KIND, bool COUNT>
 cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first,
                         bool after_trace, const LaunchPlan &plan, cudaStream_t stream,
