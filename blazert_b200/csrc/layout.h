@@ -69,7 +69,9 @@ constexpr int kVertexDoubles = 4;
 // is hit.  (The image can also be built with leaf records in place of these positions, refs then
 // being kLeafBit | the record's offset in 16-byte units: the box (lo.x, hi.x, lo.y, hi.y, lo.z,
 // hi.z; 48 B), u32 first leaf-ordered position, u32 count, 8 B zero; then the leaf's primitives,
-// triangles {i0, i1, i2, 0}, spheres and planes their payload records.)
+// triangles {i0, i1, i2, 0}, spheres and planes their payload records.  Such an image holds all
+// that a walk on the host needs, and the walk's host code reads it through KindView::leaves; no
+// scene uploads it.)
 constexpr int kWideMax = 8;
 // Entries of the thread-local traversal stack; trees whose stack needs more (depth > 62,
 // reachable only with max_tree_depth above 62) trace with the stack in shared memory in FP64,
@@ -102,6 +104,10 @@ struct KindView {
   uint32_t n_wide = 0;
   uint32_t wide_root_ref = 0;            // 0 (wide root) or kLeafBit | position of a leaf root
   float coord_max = 0.0f;       // largest |coordinate| of the root box, rounded up
+  // host code only, an image with leaf records: the records (in place of leaf_box) and their
+  // 16-byte units
+  const double *leaves = nullptr;
+  uint32_t n_leaf16 = 0;
 };
 
 struct SceneView {

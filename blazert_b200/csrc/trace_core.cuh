@@ -1169,12 +1169,28 @@ template <int KIND, bool COUNT, class F>
 BZR_HD void wtrav_leaf(const KindView &K, const Ray &r, const F &f, KState &st,
                        typename F::Bound &hl, Trav &tv, uint32_t *err, Counts *cnt) {
   if (tv.post == kNoLeaf) return;
-  const uint32_t first = tv.post & kIdMask;
+  uint32_t first = tv.post & kIdMask;
   tv.post = tv.post2;
   tv.post2 = kNoLeaf;
+#if !defined(__CUDA_ARCH__)
+  const double *record = nullptr;
+  if (K.leaves) {  // an image with leaf records (layout.h)
+    if (uint64_t(first) + kLeafHeaderBytes / 16 > K.n_leaf16) {
+      flag_error(err, kErrPrimIndex);
+      tv.live = false;
+      return;
+    }
+    record = K.leaves + 2 * size_t(first);
+    std::memcpy(&first, record + 6, sizeof first);
+  }
+#endif
   const KState before = st;
   auto box_passes = [&] {
+#if defined(__CUDA_ARCH__)
     const double *b = K.leaf_box + 6 * size_t(first);
+#else
+    const double *b = record ? record : K.leaf_box + 6 * size_t(first);
+#endif
     double key;
     return box_test(ld2(b), ld2(b + 2), ld2(b + 4), r, key) && !(key > before.hit);
   };

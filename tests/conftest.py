@@ -11,6 +11,12 @@ if ROOT not in sys.path:
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200); run with -m gpu")
+    if not hasattr(config, "workerinput"):  # once, before any worker process loads it
+        from tests.emu.emu import build as build_emu
+        try:
+            build_emu()
+        except (OSError, subprocess.CalledProcessError):
+            pass  # the tests that need the emulator say why
 
 
 @pytest.fixture(scope="session", autouse=True)
