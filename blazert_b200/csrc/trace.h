@@ -174,9 +174,9 @@ int trace_passes(const SceneView &S);
 // or null): when given, the counting kernels add per kind the box tests (totals[0..3]) and
 // primitive tests (totals[4..7]) of every ray.
 // A pass of a kind whose wide image exists is three kernels: the binary walk of the rays that the
-// wide walk leaves out (FP32: a direction component of 0 or below 2^-40 in magnitude, a tmin
-// beyond 1e18, NaN; FP64: RayD), beside it the wide walk of the others, then the binary walk of
-// those that the wide walk hands on.
+// wide walk leaves out (FP32: a direction component of 0, below 2^-40 or above 2^100 in magnitude,
+// a tmin beyond 1e18, NaN; FP64: RayD), beside it the wide walk of the others, then the binary
+// walk of those that the wide walk hands on.
 cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const LaunchPlan &plan,
                          cudaStream_t stream, uint32_t *counters,
                          unsigned long long *totals = nullptr);

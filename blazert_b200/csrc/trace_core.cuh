@@ -661,11 +661,14 @@ BZR_HD bool traverse(const KindView &K, const Ray &r, KState &st, const Stack &s
 // distance above the reference's: one grid cell of slack on top of the outward quantisation.
 // The bound follows the ray's own magnitudes on each axis: an axis whose direction component
 // is tiny has large distances and a large E, but those distances rarely decide the entry or
-// the exit.  Rays with a zero, non-finite or large (> 2^40) inverse direction component, an
-// origin component beyond 1e18, or a non-finite or huge tmin or a NaN tmax, take the FP64
+// the exit.  Rays with a zero, non-finite, large (> 2^40) or small (< 2^-100) inverse direction
+// component, an origin component beyond 1e18, or a non-finite or huge tmin or a NaN tmax, take the FP64
 // traversal.  Then every FP32 value of the test is finite: node coordinates are within 1e18
 // (the builder's limit), so 2^e <= 2^54, |A| <= 2^94, 2^23 |A| <= 2^117, |B| <= 2^101, and
-// every distance and difference stays below 2^121.
+// every distance and difference stays below 2^121.  And inv_f is a normal number, rounded within
+// 2^-24 of the FP64 inverse as the bound has it: a denormal one (a raw direction beyond 2^126) has
+// fewer bits and loses hits where coordinates are large (1e9 and more).  A and B may still be
+// denormal; their absolute errors of 2^-150, times 2^23 at most, are within the 1e-37.
 struct RayW {
   using Bound = float;
   float o_hi[3], o_lo[3], inv[3];
@@ -725,10 +728,10 @@ BZR_HD bool in_range(double x, int lo, int hi) {
   return e - (uint32_t(1023 + lo) << 20) < (uint32_t(hi - lo) << 20);
 }
 BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayW *) {
-  bool in = in_range(w[0], -39, 1000) && in_range(w[1], -39, 1000) && in_range(w[2], -39, 1000);
+  bool in = in_range(w[0], -39, 100) && in_range(w[1], -39, 100) && in_range(w[2], -39, 100);
   if (!in) {
     in = true;
-    for (int a = 0; a < 3; ++a) in = in && fabs(1.0 / w[a]) > 0.0 && fabs(1.0 / w[a]) <= 0x1p40;
+    for (int a = 0; a < 3; ++a) in = in && fabs(1.0 / w[a]) >= 0x1p-100 && fabs(1.0 / w[a]) <= 0x1p40;
   }
   return !(in && fabs(tmin) <= 1e18 && !isnan(tmax));
 }
@@ -738,7 +741,7 @@ BZR_HD RayW make_ray_f(const Ray &r, const RayW *) {
   bool ok = fabs(r.tmin) <= 1e18 && !isnan(r.tmax);
   for (int a = 0; a < 3; ++a) {
     const double ai = fabs(inv[a]), oa = fabs(o[a]);
-    ok = ok && ai > 0.0 && ai <= 0x1p40 && oa <= 1e18;  // false for NaN and infinities
+    ok = ok && ai >= 0x1p-100 && ai <= 0x1p40 && oa <= 1e18;  // false for NaN and infinities
     f.o_hi[a] = static_cast<float>(o[a]);
     f.o_lo[a] = static_cast<float>(o[a] - static_cast<double>(f.o_hi[a]));
     f.inv[a] = static_cast<float>(inv[a]);
