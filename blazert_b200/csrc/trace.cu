@@ -287,12 +287,12 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
   uint32_t n = io.n, n_uncovered = 0;
   bool scan = false, all = false;
   if constexpr (kRest) {
-    n_uncovered = *io.uncovered_count;
-    const uint32_t n_redo = *io.redo_count;
+    n_uncovered = __shfl_sync(kFull, *io.uncovered_count, 0);  // the same for every lane
+    const uint32_t n_redo = __shfl_sync(kFull, *io.redo_count, 0);
     all = n_redo > kRedoList;
     scan = all || n_uncovered > kUncoveredList;
     n = all ? io.n : scan ? io.n + n_redo : n_uncovered + n_redo;
-    if (n == 0) return;  // the same for every thread of the grid
+    if (n == 0) return;
   }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
@@ -326,19 +326,19 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
           const uint32_t rank = __popc(idle & below);
           const uint32_t idx = rank < avail ? pool_next + rank : base + (rank - avail);
           if (idx < n) {
+            active = true;
             if constexpr (kRest) {
-              const uint32_t rays = scan ? io.n : n_uncovered;
-              i = idx >= rays ? io.redo[idx - rays]
-                  : !scan     ? io.uncovered[idx]
-                  : io.perm   ? io.perm[idx]
-                              : idx;
+              i = handed_on_ray(idx, scan ? io.n : n_uncovered, scan, io.uncovered, io.redo,
+                                io.perm, io.n, io.error_word);
+              if (i == kNoRay) active = false, skipped = true;
             } else {
               i = io.perm ? io.perm[idx] : idx;
             }
-            active = true;
-            r = make_ray(io.org + 3 * size_t(i), io.dir + 3 * size_t(i),
-                         io.tmin ? io.tmin[i] : 0.0, io.tmax ? io.tmax[i] : kDblMax);
-            r.any_hit = io.any_hit != 0;
+            if (!kRest || active) {
+              r = make_ray(io.org + 3 * size_t(i), io.dir + 3 * size_t(i),
+                           io.tmin ? io.tmin[i] : 0.0, io.tmax ? io.tmax[i] : kDblMax);
+              r.any_hit = io.any_hit != 0;
+            }
             if constexpr (kWide) {
               f = make_ray_f(r, static_cast<const F *>(nullptr));
               if (f.ok) {
@@ -352,7 +352,7 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
             } else {
               if constexpr (kRest) {  // the wide pass has traced the others
                 const double *w = io.dir + 3 * size_t(i);
-                if (scan && !all && idx < io.n &&
+                if (active && scan && !all && idx < io.n &&
                     (io.wide_mode == kModeMixed
                          ? left_out(w, r.tmin, r.tmax, static_cast<const RayW *>(nullptr)) ||
                                make_ray_f(r, static_cast<const RayW *>(nullptr)).ok

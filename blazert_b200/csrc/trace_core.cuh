@@ -863,6 +863,24 @@ BZR_HD RayD make_ray_f(const Ray &r, const RayD *) {
   return f;
 }
 
+// The ray that entry idx of the binary pass after a wide one stands for: of its first `rays`
+// entries either each ray of the batch (scan, in the order perm when given) or the uncovered list,
+// then the list of rays to redo.  The lists lie in words that a later call may use again, so an
+// index past the batch's n rays is flagged and left out (kNoRay), like every other index that a
+// kernel reads from memory.
+constexpr uint32_t kNoRay = 0xFFFFFFFFu;
+BZR_HD uint32_t handed_on_ray(uint32_t idx, uint32_t rays, bool scan, const uint32_t *uncovered,
+                              const uint32_t *redo, const uint32_t *perm, uint32_t n,
+                              uint32_t *err) {
+  const uint32_t i = idx >= rays ? redo[idx - rays]
+                     : !scan     ? uncovered[idx]
+                     : perm      ? perm[idx]
+                                 : idx;
+  if (i < n) return i;
+  flag_error(err, kErrRayIndex);
+  return kNoRay;
+}
+
 // Next stack entry of the wide walk (entries carry no distance).
 BZR_HD void wtrav_pop(Trav &tv, const Stack &sk, uint32_t tid) {
   if (tv.sp > 0) {
