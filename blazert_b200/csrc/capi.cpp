@@ -41,14 +41,17 @@ int cuda_fail(cudaError_t e, const char *what) {
 // Allocations left before the injected failure (bzr_debug_fail_allocation); 0: none armed.
 std::atomic<int64_t> g_alloc_countdown{0};
 
-// Per-call device words: kSlots slots of kSlotWords = launch_trace's words (kTraceWords), whose
-// word kTraceCounterWords is the call's error word; one sticky error word for device-array calls
-// follows the slots, then the block count and the error word of small host-array batches (both
-// zero between calls).
-constexpr int kSlots = 256;
+// Per-call device words: slots of kSlotWords = launch_trace's words (kTraceWords), whose word
+// kTraceCounterWords is the call's error word.  Calls take the first kSlots in turn, each waiting
+// on the device for the call that had the slot before it (CallWords); captured calls take the
+// next kCapturedSlots, so that a replay shares its words with no call that runs beside it (up to
+// kCapturedSlots captured calls of a scene).  One sticky error word for device-array calls follows
+// the slots, then the block count and the error word of small host-array batches (both zero
+// between calls).
+constexpr int kSlots = 256, kCapturedSlots = 256;
 constexpr int kSlotWords = (bzr::kTraceWords + 15) / 16 * 16;
 static_assert(bzr::kTraceCounterWords < bzr::kTraceListWord, "slot layout");
-constexpr int kStickyWord = kSlots * kSlotWords;
+constexpr int kStickyWord = (kSlots + kCapturedSlots) * kSlotWords;
 constexpr int kSmallWords = kStickyWord + 1;
 constexpr int kDeviceWords = kSmallWords + 2;
 // Host-array batches: split into at most host_chunks (default kHostChunks, at most kMaxChunks)
@@ -144,7 +147,11 @@ struct bzr_scene {
   bzr::LaunchPlan plan;
   bool sort_possible = false;  // finite scene bounds: the coherence sort can be used
   uint32_t *slots = nullptr;  // see kSlots
-  std::atomic<uint32_t> next_slot{0};
+  std::atomic<uint32_t> next_slot{0}, next_captured{0};
+  struct SlotGuard {
+    std::mutex mu;               // held while a call that uses the slot is submitted
+    cudaEvent_t done = nullptr;  // the end of that call
+  } slot_guard[kSlots];
   // host-pointer calls: staging buffers (grown on demand) and a private stream
   std::mutex stage_mu;
   void *stage_dev = nullptr;
@@ -180,6 +187,8 @@ struct bzr_scene {
       if (copy_out) cudaStreamSynchronize(copy_out);
       cudaFree(arena);
       cudaFree(slots);
+      for (SlotGuard &g : slot_guard)
+        if (g.done) cudaEventDestroy(g.done);
       cudaFree(stage_dev);
       cudaFreeHost(pinned_err);
       cudaFreeHost(small_pin);
@@ -200,6 +209,50 @@ struct bzr_scene {
     g_ring.scene_gone();
   }
 };
+
+namespace {
+// The device words of one call on `st`, from take() until the call's kernels are queued.  The
+// words of an earlier call that may still be running are taken only behind it: the stream waits
+// for that call's end.  (The wait and the record cost the host about 2 us a call.)
+class CallWords {
+ public:
+  CallWords(bzr_scene *s, cudaStream_t st) : s_(s), st_(st) {}
+  ~CallWords() {
+    if (guard_) cudaEventRecord(guard_->done, st_);
+  }
+  CallWords(const CallWords &) = delete;
+  CallWords &operator=(const CallWords &) = delete;
+  cudaError_t take() {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st_, &cs) != cudaSuccess) {
+      cudaGetLastError();  // the call's first operation on the stream reports it
+      cs = cudaStreamCaptureStatusNone;
+    }
+    if (cs != cudaStreamCaptureStatusNone) {
+      words_ = s_->slots +
+               size_t(kSlotWords) * (kSlots + s_->next_captured.fetch_add(1) % kCapturedSlots);
+      return cudaSuccess;
+    }
+    const uint32_t slot = s_->next_slot.fetch_add(1) % kSlots;
+    bzr_scene::SlotGuard &g = s_->slot_guard[slot];
+    lock_ = std::unique_lock<std::mutex>(g.mu);
+    const cudaError_t e = g.done ? cudaStreamWaitEvent(st_, g.done, 0)
+                                 : cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    guard_ = &g;
+    words_ = s_->slots + size_t(kSlotWords) * slot;
+    return cudaSuccess;
+  }
+  uint32_t *words() const { return words_; }
+
+ private:
+  bzr_scene *s_;
+  cudaStream_t st_;
+  std::unique_lock<std::mutex> lock_;
+  bzr_scene::SlotGuard *guard_ = nullptr;
+  uint32_t *words_ = nullptr;
+};
+}  // namespace
 
 namespace bzr {
 int scene_handles(const bzr_scene *s, SceneHandles *out) {
@@ -598,7 +651,7 @@ static int staged_wait_result(bzr_scene *s, int rc) {
 static int run_small(bzr_scene *s, size_t n, const double *org, const double *dir,
                      const double *tmin, const double *tmax, double *t, double *uv, double *normal,
                      uint32_t *prim, uint32_t *geom, uint8_t *hit, int mode, bzr::RayIO io,
-                     uint32_t *counters, unsigned long long *totals) {
+                     unsigned long long *totals) {
   struct Piece {
     size_t bytes, off;
   };
@@ -687,8 +740,11 @@ static int run_small(bzr_scene *s, size_t n, const double *org, const double *di
       plan.blocks[k] = std::max(1, std::min(plan.blocks[k], need_blocks));
       plan.blocks32[k] = std::max(1, std::min(plan.blocks32[k], need_blocks));
     }
-    cudaError_t e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = bzr::launch_trace(s->view, ci, mode, plan, st, counters, totals);
+    CallWords words(s, st);
+    cudaError_t e = words.take();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+      e = bzr::launch_trace(s->view, ci, mode, plan, st, words.words(), totals);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(h + out_begin, d + out_begin, out_bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
@@ -822,13 +878,15 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
     io.geom = static_cast<uint32_t *>(out_at(4));
     io.hit = static_cast<uint8_t *>(out_at(5));
     io.error_word = reinterpret_cast<uint32_t *>(d + l.err);
-    uint32_t *words = s->slots + kSlotWords * (s->next_slot.fetch_add(1) % kSlots);
     cudaStream_t st = s->streams[c % kStreams];
+    CallWords words(s, st);
     const size_t q = c % slots;
     cudaError_t e = cudaMemcpyAsync(d, h, l.err + 256, cudaMemcpyHostToDevice, s->copy_in);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_in[q], s->copy_in);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s->ev_in[q], 0);
-    if (e == cudaSuccess) e = bzr::launch_trace(s->view, io, mode, plan, st, words, nullptr);
+    if (e == cudaSuccess) e = words.take();
+    if (e == cudaSuccess)
+      e = bzr::launch_trace(s->view, io, mode, plan, st, words.words(), nullptr);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_done[q], st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s->copy_out, s->ev_done[q], 0);
     if (e == cudaSuccess)
@@ -908,8 +966,6 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
       if (one_ray && p != org && p != dir && p != t) continue;
       n_dev += is_device_ptr(p) ? 1 : 0;
     }
-  const uint32_t slot = s->next_slot.fetch_add(1) % kSlots;
-  uint32_t *counters = s->slots + kSlotWords * slot;
   bzr::RayIO io;
   io.n = static_cast<uint32_t>(n);
   io.any_hit = (ray_flags & BZR_RAY_ANY_HIT) ? 1 : 0;
@@ -924,7 +980,11 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
       e = bzr::pool_malloc(&io.t, 8 * n, s->plan.pool, st);
       if (e != cudaSuccess) return fail(BZR_ENOMEM, "distance scratch allocation failed");
     }
-    e = bzr::launch_trace(s->view, io, mode, s->plan, st, counters, totals);
+    CallWords words(s, st);
+    // (the one launch of a small batch uses none)
+    if (totals || !bzr::small_batch(s->view, s->plan, io.n)) e = words.take();
+    if (e == cudaSuccess)
+      e = bzr::launch_trace(s->view, io, mode, s->plan, st, words.words(), totals);
     if (!t) cudaFreeAsync(io.t, st);
     return e == cudaSuccess ? BZR_OK : cuda_fail(e, "kernel launch");
   }
@@ -936,7 +996,7 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
   if (const int rc = settle_staging(s)) return rc;
   if (n <= kSmallBatch)
     return run_small(s, n, org, dir, tmin, tmax, t, uv, normal, prim, geom, hit, mode, io,
-                     counters, totals);
+                     totals);
   // chunks on the round-robin streams may run side by side on smaller grids, so that one
   // chunk's tail idles only its share of the SMs
   bzr::LaunchPlan chunk_plan = s->plan;
@@ -1013,7 +1073,9 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
   for (size_t c = 0; c < nchunks && e == cudaSuccess; ++c) {
     const size_t a = bounds[c], m = bounds[c + 1] - a;
     cudaStream_t st = s->streams[c % kStreams];
-    uint32_t *cnt = c == 0 ? counters : s->slots + kSlotWords * (s->next_slot.fetch_add(1) % kSlots);
+    CallWords words(s, st);
+    if ((e = words.take()) != cudaSuccess) break;
+    uint32_t *cnt = words.words();
     auto h2d = [&](double *dst, const double *src, size_t per) {
       if (src && e == cudaSuccess)
         e = cudaMemcpyAsync(dst + per * a, src + per * a, 8 * per * m, cudaMemcpyHostToDevice,
