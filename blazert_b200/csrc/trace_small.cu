@@ -165,20 +165,27 @@ __global__ void __maxnreg__(kRegs)
       default: write_result<kCylinders>(S, io, r, p, i); break;
     }
   }
-  if (args.done.flag) {  // results in host memory: tell the host when all of them are there
-    if (warp == 0) __threadfence_system();  // the warp that wrote the results
+  // Results in host memory: tell the host when all of them are there.  The barrier orders the
+  // block's results and error bits, of every warp, before its thread 0; the fence there, for the
+  // whole system, orders them before the block's count (or, for a lone block, the flag); and the
+  // last block's fence after the counts orders every block's before the flag, which the host reads
+  // with acquire.
+  if (args.done.flag) {
     __syncthreads();
     if (threadIdx.x == 0) {
+      unsigned long long err = gridDim.x == 1 ? atomicExch(io.error_word, 0u) : 0u;
+      __threadfence_system();
       bool last = gridDim.x == 1;
       if (!last && atomicAdd(args.done.blocks, 1u) == gridDim.x - 1) {
-        __threadfence();
+        __threadfence_system();
+        err = atomicExch(io.error_word, 0u);
         *args.done.blocks = 0;
         last = true;
       }
-      if (last) {
-        const unsigned long long err = atomicExch(io.error_word, 0u);
-        *static_cast<volatile unsigned long long *>(args.done.flag) = err << 32 | args.done.value;
-      }
+      if (last)
+        asm volatile("st.relaxed.sys.u64 [%0], %1;" ::"l"(args.done.flag),
+                     "l"(err << 32 | args.done.value)
+                     : "memory");
     }
   }
 }
