@@ -123,6 +123,26 @@ __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The wide kernel of a pass runs beside the pass's first kernel, so it does not wait for that
+// one's end, and a launch permitted by launch_dependents carries no memory ordering.  What it
+// reads of earlier kernels (closest distances, the sort's order, counters) reaches it by a release
+// and an acquire instead: a thread of the first kernel that has passed griddep_wait, and so sees
+// all of it, sets *begun; one thread of each wide block reads that, and the block's barrier passes
+// it on.  Every block of the first kernel has stored it before the wide one may launch, so nothing
+// is waited for but the store's own way; the loop's limit (a second or so) is for a word that
+// nothing set, and the block then traces nothing.
+constexpr int kBegunPolls = 1 << 20;
+__device__ __forceinline__ void begun_release(uint32_t *begun) {
+  asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(begun), "r"(1u) : "memory");
+}
+__device__ __forceinline__ bool begun_acquire(const uint32_t *begun) {
+  uint32_t v = 0;
+  if (threadIdx.x == 0)
+    for (int k = 0; !v && k < kBegunPolls; ++k)
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(begun) : "memory");
+  return __syncthreads_or(int(v));
+}
+
 // One kind over the whole batch.  first: this pass writes the whole output record.
 // COUNT: also sums the work counters into totals[16] (per kind: box tests, primitive tests,
 // node fetches, leaf fetches; see Counts).  F: NoWalk, the binary FP64 traversal; RayW or RayD,
@@ -162,6 +182,8 @@ __global__ void __launch_bounds__(kMaxTraceThreads)
   Counts cnt = {};
   // The wide kernel starts once every block is here, with whatever preceded this pass complete.
   griddep_wait();
+  if (threadIdx.x == 0) begun_release(io.begun);
+  __syncthreads();  // the store of every block comes before the launch
   griddep_launch_dependents();
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -278,9 +300,15 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
     sk.n_top = n_top;
   }
   // Up to here only the scene was read; the counters, the rays' closest distances and the
-  // lists come from earlier kernels of the stream.  (What precedes a wide kernel's first kernel
-  // is complete, and these two trace different rays; see the end.)
-  if constexpr (!kWide) griddep_wait();
+  // lists come from earlier kernels of the stream.  (A wide kernel and the first one of its pass
+  // trace different rays; see the end.)
+  if constexpr (!kWide) {
+    griddep_wait();
+  } else if (!begun_acquire(io.begun)) {
+    if (threadIdx.x == 0) flag_error(io.error_word, kErrOrder);
+    griddep_wait();
+    return;
+  }
   // The rays of a Rest pass: the listed ones, or every ray that the wide walk does not cover
   // when they outgrew their list, or every ray when those to redo outgrew theirs (a ray the
   // wide walk has finished gives the same result again).
@@ -833,6 +861,7 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
       RayIO wide = io;
       wide.uncovered_count = counters + 2 * kNumKinds + KIND;
       wide.redo_count = counters + 3 * kNumKinds + KIND;
+      wide.begun = counters + 4 * kNumKinds + KIND;
       wide.uncovered = counters + kTraceListWord;
       wide.redo = wide.uncovered + kUncoveredList;
       wide.wide_mode = mode;

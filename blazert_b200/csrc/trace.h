@@ -16,11 +16,11 @@ constexpr int kModeFp64 = 0;   // BZR_MODE_FP64
 constexpr int kModeMixed = 1;  // BZR_MODE_MIXED
 // Device words launch_trace takes per call.  First kTraceCounterWords zeroed words: the work
 // counter of each kind's pass, then for each kind the work counter of the binary pass over the
-// rays its wide walk handed on, the count of those it did not cover and the count of those whose
-// walk ended without a result.  From kTraceListWord on, the first kUncoveredList and kRedoList
+// rays its wide walk handed on, the count of those it did not cover, the count of those whose
+// walk ended without a result, and the word by which its first kernel lets the wide one begin.  From kTraceListWord on, the first kUncoveredList and kRedoList
 // of these rays' indices (the kinds' passes use them one after the other).  Words in between
 // belong to the caller.
-constexpr int kTraceCounterWords = 4 * kNumKinds;
+constexpr int kTraceCounterWords = 5 * kNumKinds;
 constexpr int kTraceListWord = kTraceCounterWords + 4;
 constexpr uint32_t kUncoveredList = 96, kRedoList = 32;
 constexpr int kTraceWords = kTraceListWord + int(kUncoveredList + kRedoList);
@@ -52,6 +52,7 @@ struct RayIO {
   // again.  Set by launch_trace.
   uint32_t *uncovered_count = nullptr, *redo_count = nullptr;
   uint32_t *uncovered = nullptr, *redo = nullptr;
+  uint32_t *begun = nullptr;  // set by the pass's first kernel once what precedes it is visible
   int wide_mode = 0;  // the mode whose wide pass handed the rays on (its cover test)
 };
 
