@@ -1005,7 +1005,7 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
   chunk_plan.early_launch = false;
   for (int k = 0; k < bzr::kNumKinds; ++k)
     for (int *b : {&chunk_plan.blocks[k], &chunk_plan.blocks32[k], &chunk_plan.blocks64w[k],
-                   &chunk_plan.blocks_out[k], &chunk_plan.blocks_rest[k]})
+                   &chunk_plan.blocks_rest[k]})
       *b = std::max(1, *b / s->host_grid_div);
   if (!totals) {
     bool pageable = false;

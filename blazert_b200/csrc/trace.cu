@@ -123,32 +123,12 @@ __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// The wide kernel of a pass runs beside the pass's first kernel, so it does not wait for that
-// one's end, and a launch permitted by launch_dependents carries no memory ordering.  What it
-// reads of earlier kernels (closest distances, the sort's order, counters) reaches it by a release
-// and an acquire instead: a thread of the first kernel that has passed griddep_wait, and so sees
-// all of it, sets *begun; one thread of each wide block reads that, and the block's barrier passes
-// it on.  Every block of the first kernel has stored it before the wide one may launch, so nothing
-// is waited for but the store's own way; the loop's limit (a second or so) is for a word that
-// nothing set, and the block then traces nothing.
-constexpr int kBegunPolls = 1 << 20;
-__device__ __forceinline__ void begun_release(uint32_t *begun) {
-  asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(begun), "r"(1u) : "memory");
-}
-__device__ __forceinline__ bool begun_acquire(const uint32_t *begun) {
-  uint32_t v = 0;
-  if (threadIdx.x == 0)
-    for (int k = 0; !v && k < kBegunPolls; ++k)
-      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(begun) : "memory");
-  return __syncthreads_or(int(v));
-}
-
 // One kind over the whole batch.  first: this pass writes the whole output record.
 // COUNT: also sums the work counters into totals[16] (per kind: box tests, primitive tests,
 // node fetches, leaf fetches; see Counts).  F: NoWalk, the binary FP64 traversal; RayW or RayD,
 // the wide walk in FP32 or FP64, which hands on the rays that it does not cover (f.ok) or that
 // end it without a result (kRedoLeaf); Rest, the binary traversal of those (cylinders always
-// take the binary traversal).  Keeping the binary walk out of the wide kernel keeps its
+// take the binary traversal).  Keeping the binary walk out of the wide walk's loop keeps its
 // registers for the wide walk.
 struct NoWalk {
   using Bound = float;
@@ -157,20 +137,24 @@ struct Rest {
   using Bound = float;
 };
 
-// The first kernel of a wide pass: each warp looks through its share of the batch for rays that
-// the wide walk leaves out and traces them through the binary nodes, lanes refilled as they
-// finish; the wide kernel runs beside it.  These rays start first because they can be the
-// slowest: the middle row of an image of odd height has a zero direction component, and along a
+// The first io.out_blocks blocks of a wide kernel: each warp looks through its share of the batch
+// for rays that the wide walk leaves out and traces them through the binary nodes, lanes refilled
+// as they finish; the other blocks walk the wide nodes.  These rays start first because they can be
+// the slowest: the middle row of an image of odd height has a zero direction component, and along a
 // plane of box bounds the reference's 0 * inf accepts thousands of boxes.  Traced after the wide
-// kernel instead, they added their whole time to it: 541,501 pixels of a 20,480-triangle sphere
-// 637 us, now 396; without that row 166.  (As a first phase, or a last one, inside the wide
-// kernel they cost the walk its registers: 8.4M bounce rays on a terrain 4,420 -> 4,560 to 4,850
-// us; a look through those takes about 10.)
+// walk instead, they added their whole time to it: 541,501 pixels of a 20,480-triangle sphere
+// 637 us, now 441; without that row 166.  (As a first phase, or a last one, of every block they
+// cost the walk its registers: 8.4M bounce rays on a terrain 4,420 -> 4,560 to 4,850 us; a look
+// through those takes about 10.  As a kernel of its own, which the wide one must run beside to gain
+// anything, they have more registers, 420 us for that image, but the wide kernel then reads what
+// earlier kernels wrote without a wait of its own; an acquire in its place empties the SM's L1
+// under the walks, 3 to 13 us a pass at 131,072 rays.)
 constexpr uint32_t kScan = 8;  // runs of 32 rays a warp looks at together: independent loads
+
 template <int KIND, bool COUNT, class F, bool LOCAL>
-__global__ void __launch_bounds__(kMaxTraceThreads)
-    trace_left_out_kernel(SceneView S, RayIO io, int first, uint32_t *,
-                          unsigned long long *totals) {
+__device__ __forceinline__ void trace_left_out_body(const SceneView &S, const RayIO &io, int first,
+                                                    unsigned long long *totals) {
+  griddep_launch_dependents();
   extern __shared__ __align__(16) unsigned char smem[];
   const KindView &K = S.k[KIND];
   double lkey[LOCAL ? kLocalStack : 1];
@@ -180,13 +164,9 @@ __global__ void __launch_bounds__(kMaxTraceThreads)
   init_stack<LOCAL>(sk, tid, S.stack_cap, smem, lkey, lref);
   if (!COUNT) prefetch_kind<KIND, true>(K);
   Counts cnt = {};
-  // The wide kernel starts once every block is here, with whatever preceded this pass complete.
   griddep_wait();
-  if (threadIdx.x == 0) begun_release(io.begun);
-  __syncthreads();  // the store of every block comes before the launch
-  griddep_launch_dependents();
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t warps = uint32_t(io.out_blocks) * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   // runs of 32 rays, dealt to the warps in turn (left-out rays tend to lie together), kScan runs
   // looked at together
@@ -300,15 +280,8 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
     sk.n_top = n_top;
   }
   // Up to here only the scene was read; the counters, the rays' closest distances and the
-  // lists come from earlier kernels of the stream.  (A wide kernel and the first one of its pass
-  // trace different rays; see the end.)
-  if constexpr (!kWide) {
-    griddep_wait();
-  } else if (!begun_acquire(io.begun)) {
-    if (threadIdx.x == 0) flag_error(io.error_word, kErrOrder);
-    griddep_wait();
-    return;
-  }
+  // lists come from earlier kernels of the stream.
+  griddep_wait();
   // The rays of a Rest pass: the listed ones, or every ray that the wide walk does not cover
   // when they outgrew their list, or every ray when those to redo outgrew theirs (a ray the
   // wide walk has finished gives the same result again).
@@ -371,7 +344,7 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
               f = make_ray_f(r, static_cast<const F *>(nullptr));
               if (f.ok) {
                 wtrav_begin<KIND, COUNT>(K, r, f, st, hl, tv, &cnt);
-              } else {  // the pass's first kernel has it, or it is handed on
+              } else {  // the pass's first blocks have it, or it is handed on
                 active = false;
                 skipped = true;
                 deferred = !left_out(io.dir + 3 * size_t(i), r.tmin, r.tmax,
@@ -448,7 +421,6 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
       }
     }
   }
-  if constexpr (kWide) griddep_wait();  // this grid is not complete before the pass's first one
   if (COUNT) {
     for (int k = 0; k < kNumKinds; ++k) {
       unsigned long long v[4] = {cnt.box[k], cnt.prim[k], cnt.node[k], cnt.leaf[k]};
@@ -477,7 +449,10 @@ template <int KIND, bool COUNT, bool LOCAL>
 __global__ void __maxnreg__(BZR_WIDE_REGS)
     trace_wide_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
                       unsigned long long *totals) {
-  trace_kind_body<KIND, COUNT, RayW, LOCAL>(S, io, first, work_counter, totals);
+  if (int(blockIdx.x) < io.out_blocks)
+    trace_left_out_body<KIND, COUNT, RayW, LOCAL>(S, io, first, totals);
+  else
+    trace_kind_body<KIND, COUNT, RayW, LOCAL>(S, io, first, work_counter, totals);
 }
 
 // The FP64 mode's wide walk, with the thread-local stack (other stacks take the binary walk).
@@ -489,7 +464,10 @@ template <int KIND>
 __global__ void __maxnreg__(kWide64Regs)
     trace_wide64_kernel(SceneView S, RayIO io, int first, uint32_t *work_counter,
                       unsigned long long *totals) {
-  trace_kind_body<KIND, false, RayD, true>(S, io, first, work_counter, totals);
+  if (int(blockIdx.x) < io.out_blocks)
+    trace_left_out_body<KIND, false, RayD, true>(S, io, first, totals);
+  else
+    trace_kind_body<KIND, false, RayD, true>(S, io, first, work_counter, totals);
 }
 
 // The binary pass over the rays that a wide pass handed on.
@@ -832,8 +810,8 @@ cudaError_t launch_one(TraceFn fn, int blocks, int threads, size_t smem, cudaStr
   return cudaLaunchKernelEx(&cfg, fn, S, io, first, counter, totals);
 }
 
-// The pass of one kind: one kernel, or for a wide walk three: the binary walk of the rays it leaves
-// out, beside it the wide kernel, then the binary walk of the rays that one handed on.  counters:
+// The pass of one kind: one kernel, or for a wide walk two: the wide kernel, then the binary walk of
+// the rays that one handed on.  counters:
 // the kTraceWords words of the call; after_trace: a trace kernel of this call precedes the pass on
 // the stream.
 template <int KIND, bool COUNT>
@@ -861,20 +839,13 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
       RayIO wide = io;
       wide.uncovered_count = counters + 2 * kNumKinds + KIND;
       wide.redo_count = counters + 3 * kNumKinds + KIND;
-      wide.begun = counters + 4 * kNumKinds + KIND;
       wide.uncovered = counters + kTraceListWord;
       wide.redo = wide.uncovered + kUncoveredList;
       wide.wide_mode = mode;
-      const TraceFn out_fn =
-          mixed ? (local ? trace_left_out_kernel<KIND, false, RayW, true>
-                         : trace_left_out_kernel<KIND, COUNT, RayW, false>)
-                : trace_left_out_kernel<KIND, false, RayD, true>;
-      cudaError_t e = launch_one(out_fn, grid(plan.blocks_out[KIND]), th, smem, stream, early, S,
-                                 wide, first, nullptr, totals);
-      if (e != cudaSuccess) return e;
-      e =
-          launch_one(wide_fn, grid(mixed ? plan.blocks32[KIND] : plan.blocks64w[KIND]), th,
-                     smem, stream, plan.early_launch, S, wide, first, counters + KIND, totals);
+      const int blocks = grid(mixed ? plan.blocks32[KIND] : plan.blocks64w[KIND]);
+      wide.out_blocks = blocks;
+      const cudaError_t e = launch_one(wide_fn, 2 * blocks, th, smem, stream, early, S, wide, first,
+                                       counters + KIND, totals);
       if (e != cudaSuccess) return e;
       // hardly ever any ray: a small grid, which leaves the SMs to the next pass
       return launch_one(rest_fn, grid(std::min(plan.blocks_rest[KIND], plan.sms)), th, smem, stream,
@@ -925,14 +896,6 @@ cudaError_t prepare_kind(const SceneView &S, LaunchPlan *plan) {
                                reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, false>)};
     for (const void *fn : rest_fns)
       if (e == cudaSuccess) e = grid_for(fn, th, smem, plan->sms, &plan->blocks_rest[KIND]);
-    const void *out_fns[4] = {
-        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, true, RayW, false>),
-        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayW, false>),
-        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayW, true>),
-        reinterpret_cast<const void *>(trace_left_out_kernel<KIND, false, RayD, true>)};
-    for (int j = 0; j < (local ? 4 : 2); ++j)
-      if (e == cudaSuccess)
-        e = grid_for(out_fns[j], th, j < 2 ? smem : bytes, plan->sms, &plan->blocks_out[KIND]);
     if (local && e == cudaSuccess)
       e = grid_for(reinterpret_cast<const void *>(trace_rest_kernel<KIND, false, true>), th, bytes,
                    plan->sms, &plan->blocks_rest[KIND]);

@@ -16,11 +16,11 @@ constexpr int kModeFp64 = 0;   // BZR_MODE_FP64
 constexpr int kModeMixed = 1;  // BZR_MODE_MIXED
 // Device words launch_trace takes per call.  First kTraceCounterWords zeroed words: the work
 // counter of each kind's pass, then for each kind the work counter of the binary pass over the
-// rays its wide walk handed on, the count of those it did not cover, the count of those whose
-// walk ended without a result, and the word by which its first kernel lets the wide one begin.  From kTraceListWord on, the first kUncoveredList and kRedoList
+// rays its wide walk handed on, the count of those it did not cover and the count of those whose
+// walk ended without a result.  From kTraceListWord on, the first kUncoveredList and kRedoList
 // of these rays' indices (the kinds' passes use them one after the other).  Words in between
 // belong to the caller.
-constexpr int kTraceCounterWords = 5 * kNumKinds;
+constexpr int kTraceCounterWords = 4 * kNumKinds;
 constexpr int kTraceListWord = kTraceCounterWords + 4;
 constexpr uint32_t kUncoveredList = 96, kRedoList = 32;
 constexpr int kTraceWords = kTraceListWord + int(kUncoveredList + kRedoList);
@@ -45,14 +45,14 @@ struct RayIO {
   uint32_t chunk = kRayChunk;      // rays a warp takes per fetch: 32, 64, 128, or 0 for
                                    // exactly the lanes that are idle
   uint32_t top_nodes = 0;          // top-level nodes each block stages in shared memory
-  // Wide passes: the rays that the pass's first kernel leaves to the walk but that the walk does
-  // not cover (origins beyond its range), or whose walk ends without a result, are counted here
+  // Wide passes: the rays that the first blocks leave to the walk but that the walk does not
+  // cover (origins beyond its range), or whose walk ends without a result, are counted here
   // and the first of each noted in the lists, for the binary pass right after.  A batch has
   // hardly any: a short list needs no allocation, and past it the binary pass looks at every ray
   // again.  Set by launch_trace.
   uint32_t *uncovered_count = nullptr, *redo_count = nullptr;
   uint32_t *uncovered = nullptr, *redo = nullptr;
-  uint32_t *begun = nullptr;  // set by the pass's first kernel once what precedes it is visible
+  int out_blocks = 0;  // a wide kernel's first blocks, which trace the rays its walk leaves out
   int wide_mode = 0;  // the mode whose wide pass handed the rays on (its cover test)
 };
 
@@ -80,7 +80,6 @@ struct LaunchPlan {
   int blocks[kNumKinds] = {0, 0, 0, 0};    // FP64 kernels
   int blocks32[kNumKinds] = {0, 0, 0, 0};  // mixed-precision kernels
   int blocks64w[kNumKinds] = {0, 0, 0, 0};  // the FP64 mode's wide kernels
-  int blocks_out[kNumKinds] = {0, 0, 0, 0};   // the first kernels of wide passes
   int blocks_rest[kNumKinds] = {0, 0, 0, 0};  // the binary passes after wide ones
   int small_blocks[kNumKinds] = {0, 0, 0, 0};  // resident blocks of the small kernel, by kinds
   RaySort sort;
@@ -174,10 +173,10 @@ int trace_passes(const SceneView &S);
 // counters: kTraceWords device words, zeroed here as far as needed.  totals (device, 8 x uint64,
 // or null): when given, the counting kernels add per kind the box tests (totals[0..3]) and
 // primitive tests (totals[4..7]) of every ray.
-// A pass of a kind whose wide image exists is three kernels: the binary walk of the rays that the
-// wide walk leaves out (FP32: a direction component of 0, below 2^-40 or above 2^100 in magnitude,
-// a tmin beyond 1e18, NaN; FP64: RayD), beside it the wide walk of the others, then the binary
-// walk of those that the wide walk hands on.
+// A pass of a kind whose wide image exists is two kernels: one whose first blocks run the binary
+// walk of the rays that the wide walk leaves out (FP32: a direction component of 0, below 2^-40 or
+// above 2^100 in magnitude, a tmin beyond 1e18, NaN; FP64: RayD) and whose others run the wide walk
+// of the rest, then the binary walk of those that the wide walk hands on.
 cudaError_t launch_trace(const SceneView &S, const RayIO &io, int mode, const LaunchPlan &plan,
                          cudaStream_t stream, uint32_t *counters,
                          unsigned long long *totals = nullptr);
