@@ -151,6 +151,37 @@ struct Rest {
 // under the walks, 3 to 13 us a pass at 131,072 rays.)
 constexpr uint32_t kScan = 8;  // runs of 32 rays a warp looks at together: independent loads
 
+// Whether the wide walk covers hardly any ray of a large batch (an orthographic camera along an
+// axis, a negative tmin in FP64 mode, far origins): at most 4 of 32 rays spread over it, twice.
+// Such a batch is left to the binary pass as a whole, whose persistent kernel holds more warps than
+// the blocks below and takes its rays in order; every block comes to the same answer.  1M / 4M
+// rays, by the blocks below and so: raster rays straight down on a terrain 259 / 955 and 224 / 720
+// us (the binary kernel alone 215 / 702), rays with tmin -1 in it 920 / 2,943 and 836 / 2,620.
+// 524,288 of those 629 and 608, 400,000 476 and 484; with 10,000 spheres 1M 1,015 and 1,037, 4M
+// 3,490 and 3,348.
+constexpr uint32_t kWholeMinMesh = 1u << 19, kWholeMin = 1u << 21;
+template <int KIND>
+__host__ __device__ constexpr uint32_t whole_min() {
+  return KIND == kMesh ? kWholeMinMesh : kWholeMin;
+}
+template <int KIND, class F>
+__device__ __forceinline__ bool covers_hardly_any(const RayIO &io) {
+  if (io.n < whole_min<KIND>()) return false;
+  bool hardly = false;
+  if (threadIdx.x < 32) {  // scattered loads: one warp of a block makes them
+    auto covered = [&](uint32_t j) {
+      const size_t i = (size_t(threadIdx.x) * 2 + j) * io.n / 64;
+      const F *f = nullptr;
+      const bool out = left_out(io.dir + 3 * i, io.tmin ? io.tmin[i] : 0.0,
+                                io.tmax ? io.tmax[i] : kDblMax, f) ||
+                       far_origin(io.org + 3 * i, f);
+      return __popc(__ballot_sync(kFull, !out));
+    };
+    hardly = covered(0) <= 4 && covered(1) <= 4;
+  }
+  return __syncthreads_or(hardly);
+}
+
 template <int KIND, bool COUNT, class F, bool LOCAL>
 __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const RayIO &io, int first,
                                                     unsigned long long *totals) {
@@ -166,6 +197,7 @@ __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const Ra
   Counts cnt = {};
   griddep_wait();
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  if (covers_hardly_any<KIND, F>(io)) return;
   const uint32_t warps = uint32_t(io.out_blocks) * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   // runs of 32 rays, dealt to the warps in turn (left-out rays tend to lie together), kScan runs
@@ -282,15 +314,19 @@ __device__ __forceinline__ void trace_kind_body(const SceneView &S, const RayIO 
   // Up to here only the scene was read; the counters, the rays' closest distances and the
   // lists come from earlier kernels of the stream.
   griddep_wait();
+  if constexpr (kWide)
+    if (covers_hardly_any<KIND, F>(io)) return;
   // The rays of a Rest pass: the listed ones, or every ray that the wide walk does not cover
-  // when they outgrew their list, or every ray when those to redo outgrew theirs (a ray the
-  // wide walk has finished gives the same result again).
+  // when they outgrew their list, or every ray when the wide kernel left it the whole batch or
+  // those to redo outgrew theirs (a ray the wide walk has finished gives the same result again).
   uint32_t n = io.n, n_uncovered = 0;
   bool scan = false, all = false;
   if constexpr (kRest) {
     n_uncovered = __shfl_sync(kFull, *io.uncovered_count, 0);  // the same for every lane
     const uint32_t n_redo = __shfl_sync(kFull, *io.redo_count, 0);
-    all = n_redo > kRedoList;
+    const bool whole = io.wide_mode == kModeMixed ? covers_hardly_any<KIND, RayW>(io)
+                                                  : covers_hardly_any<KIND, RayD>(io);
+    all = whole || n_redo > kRedoList;
     scan = all || n_uncovered > kUncoveredList;
     n = all ? io.n : scan ? io.n + n_redo : n_uncovered + n_redo;
     if (n == 0) return;
@@ -847,9 +883,13 @@ cudaError_t launch_kind(const SceneView &S, const RayIO &io, int mode, int first
       const cudaError_t e = launch_one(wide_fn, 2 * blocks, th, smem, stream, early, S, wide, first,
                                        counters + KIND, totals);
       if (e != cudaSuccess) return e;
-      // hardly ever any ray: a small grid, which leaves the SMs to the next pass
-      return launch_one(rest_fn, grid(std::min(plan.blocks_rest[KIND], plan.sms)), th, smem, stream,
-                        plan.early_launch, S, wide, first, counters + kNumKinds + KIND, totals);
+      // Hardly ever any ray: a small grid, which leaves the SMs to the next pass, except where it
+      // can be all of them, a large batch (covers_hardly_any) or one of far origins in mixed mode.
+      const bool few = !mixed && io.n < whole_min<KIND>();
+      const int rest_blocks = few ? std::min(plan.blocks_rest[KIND], plan.sms)
+                                  : plan.blocks_rest[KIND];
+      return launch_one(rest_fn, grid(rest_blocks), th, smem, stream, plan.early_launch, S, wide,
+                        first, counters + kNumKinds + KIND, totals);
     }
   }
   return launch_one(fp64, grid(plan.blocks[KIND]), th, smem, stream, early, S, io, first,

@@ -735,6 +735,10 @@ BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayW *) {
   }
   return !(in && fabs(tmin) <= 1e18 && !isnan(tmax));
 }
+// The origin's part of make_ray_f's ok.
+BZR_HD bool far_origin(const double *o, const RayW *) {
+  return !(fabs(o[0]) <= 1e18 && fabs(o[1]) <= 1e18 && fabs(o[2]) <= 1e18);
+}
 BZR_HD RayW make_ray_f(const Ray &r, const RayW *) {
   RayW f;
   const double inv[3] = {r.inv.x, r.inv.y, r.inv.z}, o[3] = {r.o.x, r.o.y, r.o.z};
@@ -848,6 +852,9 @@ BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayD *) {
       in = in && fabs(1.0 / w[a]) >= 0x1p-500 && fabs(1.0 / w[a]) <= 0x1p500;
   }
   return !(in && tmin >= 0.0 && !isnan(tmax));
+}
+BZR_HD bool far_origin(const double *o, const RayD *) {
+  return !(fabs(o[0]) <= 0x1p300 && fabs(o[1]) <= 0x1p300 && fabs(o[2]) <= 0x1p300);
 }
 BZR_HD RayD make_ray_f(const Ray &r, const RayD *) {
   RayD f;

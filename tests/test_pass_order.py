@@ -44,3 +44,39 @@ def test_repeated_calls_of_several_kinds(mode, sort):
         assert mismatches(got, ref) == [], rep
     assert scene.check() == 0
     scene.close()
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+@pytest.mark.parametrize("rays", ["axis", "mostly_axis", "far"])
+def test_large_batches_the_wide_walk_hardly_covers(mode, rays):
+    """Batches above the line from which a pass is left to the binary kernel as a whole when hardly
+    any of its rays is covered: all axis-parallel, all but a few (the sample may or may not meet
+    them), and far origins."""
+    import torch
+
+    n = 2_097_152 + 3_001 if mode == "fp64" and rays == "axis" else 800_003
+    v, f = W.icosphere(4)
+    mix = W.SceneSpec().add_mesh(v, f)
+    mix.add_spheres(*W.mixed_primitives(n_rays=1, n_spheres=50, seed=3).scene.spheres.values())
+    scene, ora = product_scene(mix), Oracle(mix)
+    rng = np.random.default_rng(5)
+    m = 50_021
+    o, d = rng.uniform(-1.2, 1.2, (m, 3)), np.tile([0.0, 0.0, -1.0], (m, 1))
+    o[:, 2] = 3.0
+    if rays == "mostly_axis":
+        d[::50] = rng.standard_normal((len(d[::50]), 3))
+    if rays == "far":
+        d[:] = rng.standard_normal((m, 3))
+        o = rng.uniform(-1.2, 1.2, (m, 3)) - 3e18 * d
+    ref = ora.intersect(o, d)
+    idx = torch.arange(n, device="cuda") % m
+    out = scene.intersectN(torch.from_numpy(o).cuda()[idx], torch.from_numpy(d).cuda()[idx],
+                           mode=mode)
+    idx = idx.cpu().numpy()
+    got = to_numpy(out)
+    for k in ("prim", "geom"):
+        got[k] = got[k].view(np.uint32)
+    assert mismatches(got, {k: ref[k][idx] for k in ("t", "uv", "normal", "prim", "geom",
+                                                     "hit")}) == []
+    assert scene.check() == 0
+    scene.close()
