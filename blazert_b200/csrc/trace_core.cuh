@@ -643,11 +643,14 @@ BZR_HD bool traverse(const KindView &K, const Ray &r, KState &st, const Stack &s
 // in the same relative order (the wide tree is the binary tree with treelets contracted, and a
 // treelet's children are visited in the binary order).  The FP64 traversal processes a leaf
 // iff the leaf's own test passes at its pop time AND every ancestor passed its test at its own
-// pop time.  An ancestor's box contains the leaf's box, the rounded slab distances are
-// monotone in the box bounds, and the hit distance only decreases for triangles, spheres and
-// planes (cylinders, which may move it outward, keep the FP64 traversal); so when a leaf's own
-// test passes, no ancestor failed.  The same leaves are therefore processed in the same order
-// with the same hit distance, and every primitive test and result is identical.
+// pop time.  An ancestor's box contains the leaf's box and the rounded slab distances are
+// monotone in the box bounds, so where an ancestor failed, the first leaf under it fails at the
+// same hit distance, which that leaves as it was for the next one.  The same leaves are therefore
+// processed in the same order with the same hit distance, and every primitive test and result is
+// identical.  A child may be tested long before the reference's walk comes to it, against the
+// bound of that time: no later hit distance may exceed a bound that was in use, or the ray is
+// traced again by the binary walk (kRedoLeaf; cylinders, whose hits need not be closer than the
+// one before, always take it).
 //
 // Error bound, per node and axis: with A = 2^e inv_f, D = (origin - o_hi) - o_lo (the origin
 // held as two floats, so it is exact to 2^-48 relative), B = D inv_f and C = B - 2^23 A, the
@@ -774,10 +777,11 @@ BZR_HD RayW make_ray_f(const Ray &r, const RayW *) {
 //
 // Two things end a wide walk without a result; such a ray is traced again by the binary walk
 // (kRedoLeaf, and rays whose f.ok is false before they start):
-//  * a hit that moves the hit distance outward.  A sphere's distance norm(t d) and a triangle's
-//    t * (1 / |det|) are rounded after the comparison with the current distance and can exceed
-//    it by an ulp, and a sphere hit behind the origin (tmin < 0) is reported at its absolute
-//    distance; the argument needs distances that never grow.
+//  * a hit beyond the bound that the child tests have used (walk_bound).  A sphere's distance
+//    norm(t d) and a triangle's t * (1 / |det|) are rounded after the comparison with the current
+//    distance and can exceed it by a few ulps: the bound allows for them, so that neither
+//    coplanar triangles nor touching spheres end a walk.  A sphere or plane hit behind the origin
+//    (tmin < 0, FP32 only) is reported at its absolute distance, which can be any.
 //  * a zero or non-finite direction component, where a slab distance may be NaN and is not
 //    monotone in the bound.
 //
@@ -844,6 +848,17 @@ BZR_HD float hit_bound(const RayW &, double h) {
 }
 BZR_HD int32_t hit_bound(const RayD &, double h) { return h == 0.0 ? 0 : hi_word(h); }
 
+// The bound that the walk's child tests use for hit distance h: of h and 2^-40 of it, far more
+// than a later hit exceeds it by in rounding and far less than a child test resolves.
+template <class F>
+BZR_HD typename F::Bound walk_bound(const F &f, double h) {
+#if defined(__CUDA_ARCH__)
+  return hit_bound(f, __fma_rn(fabs(h), 0x1p-40, h));
+#else
+  return hit_bound(f, fma(fabs(h), 0x1p-40, h));
+#endif
+}
+
 BZR_HD bool left_out(const double *w, double tmin, double tmax, const RayD *) {
   bool in = in_range(w[0], -499, 499) && in_range(w[1], -499, 499) && in_range(w[2], -499, 499);
   if (!in) {
@@ -907,7 +922,7 @@ BZR_HD void wtrav_begin(const KindView &K, const Ray &r, const F &f, KState &st,
   tv.cur = K.wide_root_ref;
   tv.post = tv.post2 = kNoLeaf;
   tv.walk = tv.live;
-  hl = hit_bound(f, st.hit);
+  hl = walk_bound(f, st.hit);
 }
 
 // prmt.b32 in its default mode: byte i of the result is byte (s_i & 7) of the eight bytes
@@ -1253,12 +1268,13 @@ BZR_HD void wtrav_leaf(const KindView &K, const Ray &r, const F &f, KState &st,
           tv.live = false;
           return;
         }
-        if (!(st.hit <= before.hit)) {  // moved outward, or NaN (see RayD)
+        if (isnan(st.hit) || !(hit_bound(f, st.hit) <= hl)) {  // beyond the bound (see RayD)
           tv.post = kRedoLeaf;
           tv.live = false;
           return;
         }
-        hl = hit_bound(f, st.hit);
+        const typename F::Bound b = walk_bound(f, st.hit);
+        hl = b < hl ? b : hl;
       }
     }
   }
