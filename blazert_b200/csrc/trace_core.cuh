@@ -1268,7 +1268,8 @@ BZR_HD void wtrav_leaf(const KindView &K, const Ray &r, const F &f, KState &st,
           tv.live = false;
           return;
         }
-        if (isnan(st.hit) || !(hit_bound(f, st.hit) <= hl)) {  // beyond the bound (see RayD)
+        // beyond the bound (see RayD); the distance before is within it
+        if (!(st.hit <= before.hit) && (isnan(st.hit) || !(hit_bound(f, st.hit) <= hl))) {
           tv.post = kRedoLeaf;
           tv.live = false;
           return;
