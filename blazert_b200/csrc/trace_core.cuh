@@ -1238,7 +1238,14 @@ BZR_HD void wtrav_leaf(const KindView &K, const Ray &r, const F &f, KState &st,
     return box_test(ld2(b), ld2(b + 2), ld2(b + 4), r, key) && !(key > before.hit);
   };
   // the counting kernels test it first, as the reference does, so that they count its tests
-  if (COUNT) cnt->leaf[KIND] += 1;
+  if (COUNT) {
+    if (first >= K.n_prims) {
+      flag_error(err, kErrPrimIndex);
+      tv.live = false;
+      return;
+    }
+    cnt->leaf[KIND] += 1;
+  }
   if (!COUNT || box_passes()) {
     bool any = false;
     for (uint32_t pos = first;; ++pos) {
