@@ -66,9 +66,10 @@ constexpr size_t kMinChunk = size_t(1) << 17;
 constexpr size_t kSmallBatch = 4096;
 // Large batches from pageable host memory pass through a ring of kStageSlots pinned blocks of
 // kStageRays rays each (run_staged).  Blocks of 32k / 64k / 128k rays: 1,048,576 rays in 7.5 /
-// 5.5 / 5.3 ms, and pinning the ring takes about 1 ms per MB once (10 / 20 / 41 MB).  Batches of
-// less than kStagedMin rays keep the driver's copies: 131,073 rays 1.5 ms against 1.2, 200,000
-// rays 2.3 against 1.7.
+// 5.5 / 5.3 ms, and pinning the ring takes about 1 ms per MB once (12 / 24 / 48 MB).  Batches that
+// do not fill the ring keep the driver's copies.  Those and the ring, in ms (fresh or reused result
+// arrays, from run to run): 131,073 rays 1.0 to 1.1 and 0.6 to 1.1, 160,000 1.2 to 1.3 and 0.6 to
+// 1.1, 200,000 1.4 to 1.6 and 0.8 to 1.1.
 constexpr size_t kStageSlots = 3;
 constexpr size_t kStageRays = size_t(1) << 16;
 constexpr size_t kStagedMin = kStageSlots * kStageRays;
@@ -791,12 +792,15 @@ static int wait_event(cudaEvent_t ev, int timeout_ms) {
 // the threads unpack them, while the next chunks are on their way.  What is left is the host's
 // own copying (and the page faults of fresh result arrays), which the threads share.
 // 1,048,576 rays through three kinds, plain numpy arrays: 18.1 -> 5.5 ms.
-// A block: org, dir, [tmin], [tmax], the error word, the requested outputs, and t at the end
-// when it was not requested; each piece 256-byte aligned.  Returns kNoRing when the ring is lent
-// or cannot be allocated (the caller then lets the driver copy).
+// Arrays that the caller pinned go straight between their place and the device, beside the block.
+// A block: the pageable ones of org, dir, [tmin], [tmax], the error word, the pageable ones of
+// the requested outputs; on the device only, the pinned inputs and outputs after them, and t when
+// it was not requested; each piece 256-byte aligned.  Returns kNoRing when the ring is lent or
+// cannot be allocated (the caller then lets the driver copy).
 constexpr int kNoRing = 1;
 static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *const outs[6],
-                      int mode, int any_hit, const bzr::LaunchPlan &plan) {
+                      const bool in_ring[4], const bool out_ring[6], int mode, int any_hit,
+                      const bzr::LaunchPlan &plan) {
   static constexpr size_t kIn[4] = {24, 24, 8, 8}, kOut[6] = {8, 16, 24, 4, 4, 1};
   const size_t nchunks = (n + kStageRays - 1) / kStageRays;
   const size_t chunk = (n + nchunks - 1) / nchunks;
@@ -807,17 +811,27 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
   auto layout = [&](size_t m) {
     Layout l;
     size_t at = 0;
-    for (int j = 0; j < 4; ++j) {
-      l.in[j] = at;
-      if (ins[j]) at += align_up(kIn[j] * m, 256);
-    }
+    auto inputs = [&](bool ring) {
+      for (int j = 0; j < 4; ++j)
+        if (ins[j] && in_ring[j] == ring) {
+          l.in[j] = at;
+          at += align_up(kIn[j] * m, 256);
+        }
+    };
+    auto outputs = [&](bool ring) {
+      for (int j = 0; j < 6; ++j)
+        if (outs[j] && out_ring[j] == ring) {
+          l.out[j] = at;
+          at += align_up(kOut[j] * m, 256);
+        }
+    };
+    inputs(true);
     l.err = at;
     at += 256;
-    for (int j = 0; j < 6; ++j) {
-      l.out[j] = at;
-      if (outs[j]) at += align_up(kOut[j] * m, 256);
-    }
+    outputs(true);
     l.out_end = at;
+    inputs(false);
+    outputs(false);
     if (!outs[0]) {
       l.out[0] = at;
       at += align_up(kOut[0] * m, 256);
@@ -844,10 +858,10 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
       return fail(BZR_ENOMEM, "staging allocation failed");
     s->stage_bytes = slots * block;
   }
-  // a thread per 4 MB of the call's copies, at most eight
+  // a thread per 4 MB of the call's copies through the ring, at most eight
   size_t bytes = 0;
-  for (int j = 0; j < 4; ++j) bytes += ins[j] ? kIn[j] * n : 0;
-  for (int j = 0; j < 6; ++j) bytes += outs[j] ? kOut[j] * n : 0;
+  for (int j = 0; j < 4; ++j) bytes += ins[j] && in_ring[j] ? kIn[j] * n : 0;
+  for (int j = 0; j < 6; ++j) bytes += outs[j] && out_ring[j] ? kOut[j] * n : 0;
   bzr::CopyCrew crew(bzr::range_workers(bytes, size_t(4) << 20, 8));
   uint32_t bits = 0;
   auto submit = [&](size_t c) {
@@ -858,7 +872,7 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
     bzr::HostCopy in[4];
     size_t k = 0;
     for (int j = 0; j < 4; ++j)
-      if (ins[j])
+      if (ins[j] && in_ring[j])
         in[k++] = {h + l.in[j], static_cast<const char *>(ins[j]) + kIn[j] * a, kIn[j] * m};
     crew.run(in, k);
     std::memset(h + l.err, 0, sizeof(uint32_t));
@@ -882,6 +896,10 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
     CallWords words(s, st);
     const size_t q = c % slots;
     cudaError_t e = cudaMemcpyAsync(d, h, l.err + 256, cudaMemcpyHostToDevice, s->copy_in);
+    for (int j = 0; j < 4; ++j)
+      if (e == cudaSuccess && ins[j] && !in_ring[j])
+        e = cudaMemcpyAsync(d + l.in[j], static_cast<const char *>(ins[j]) + kIn[j] * a,
+                            kIn[j] * m, cudaMemcpyHostToDevice, s->copy_in);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_in[q], s->copy_in);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s->ev_in[q], 0);
     if (e == cudaSuccess) e = words.take();
@@ -892,6 +910,10 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(h + l.err, d + l.err, l.out_end - l.err, cudaMemcpyDeviceToHost,
                           s->copy_out);
+    for (int j = 0; j < 6; ++j)
+      if (e == cudaSuccess && outs[j] && !out_ring[j])
+        e = cudaMemcpyAsync(static_cast<char *>(outs[j]) + kOut[j] * a, d + l.out[j], kOut[j] * m,
+                            cudaMemcpyDeviceToHost, s->copy_out);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_out[q], s->copy_out);
     return e;
   };
@@ -904,7 +926,8 @@ static int run_staged(bzr_scene *s, size_t n, const void *const ins[4], void *co
     bzr::HostCopy out[6];
     size_t k = 0;
     for (int j = 0; j < 6; ++j)
-      if (outs[j]) out[k++] = {static_cast<char *>(outs[j]) + kOut[j] * a, h + l.out[j], kOut[j] * m};
+      if (outs[j] && out_ring[j])
+        out[k++] = {static_cast<char *>(outs[j]) + kOut[j] * a, h + l.out[j], kOut[j] * m};
     crew.run(out, k);
     uint32_t word;
     std::memcpy(&word, h + l.err, sizeof word);
@@ -1008,12 +1031,19 @@ static int run_batch(const bzr_scene *cs, size_t n, const double *org, const dou
                    &chunk_plan.blocks_rest[k]})
       *b = std::max(1, *b / s->host_grid_div);
   if (!totals) {
-    bool pageable = false;
-    for (const void *p : ptrs) pageable = pageable || (p && is_pageable(p));
+    bool ring[10], pageable = false;
+    for (int j = 0; j < 10; ++j) {
+      ring[j] = ptrs[j] && is_pageable(ptrs[j]);
+      // A copy out to pageable memory returns only when it is done, one in of 8 bytes a ray hardly
+      // disturbs: with pageable ranges alone the driver's copies are the faster ones (1,048,576
+      // rays 2.0 ms against 2.5).
+      pageable = pageable || (ring[j] && ptrs[j] != tmin && ptrs[j] != tmax);
+    }
     if (pageable && n >= kStagedMin) {
       const void *const ins[4] = {org, dir, tmin, tmax};
       void *const outs[6] = {t, uv, normal, prim, geom, hit};
-      const int rc = run_staged(s, n, ins, outs, mode, io.any_hit, chunk_plan);
+      const int rc =
+          run_staged(s, n, ins, outs, ring, ring + 4, mode, io.any_hit, chunk_plan);
       if (rc != kNoRing) return rc;
     }
   }
