@@ -631,6 +631,10 @@ static int settle_staging(bzr_scene *s) {
     if (rc) return rc;
   }
   s->stage_pending = false;
+  if (s->ring) {  // no work uses it any more: other scenes may have it
+    g_ring.give_back();
+    s->ring = nullptr;
+  }
   return BZR_OK;
 }
 
@@ -1726,6 +1730,11 @@ bool injected_allocation_failure() {
   return false;
 }
 }  // namespace bzr
+
+int bzr_debug_ring_lent(void) {
+  std::lock_guard<std::mutex> lock(g_ring.mu);
+  return g_ring.lent ? 1 : 0;
+}
 
 int bzr_debug_fail_allocation(int64_t k) {
   if (k < 0) return fail(BZR_EINVAL, "k must be >= 0");

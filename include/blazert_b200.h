@@ -362,6 +362,9 @@ const char *bzr_last_error_string(void);
  * hook disarms itself when it fires).  The entry point that meets the failure returns
  * BZR_ENOMEM and releases what it had allocated; the scene stays usable. */
 int bzr_debug_fail_allocation(int64_t k);
+/* Test hook: 1 while a call holds the process's pinned ring (large batches from pageable arrays), or
+ * a scene does whose call ended with work still queued. */
+int bzr_debug_ring_lent(void);
 
 #ifdef __cplusplus
 }
