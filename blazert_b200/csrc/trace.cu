@@ -521,8 +521,8 @@ __global__ void __launch_bounds__(kMaxTraceThreads)
 }
 
 template <int KIND, bool COUNT, bool MIXED, bool LOCAL>
-constexpr auto trace_kernel() {
-  if constexpr (MIXED)
+constexpr auto trace_kernel() {  // cylinders have no wide walk
+  if constexpr (MIXED && KIND != kCylinders)
     return trace_wide_kernel<KIND, COUNT, LOCAL>;
   else
     return trace_kind_kernel<KIND, COUNT, LOCAL>;
@@ -713,7 +713,7 @@ __global__ void __maxnreg__(kBatchWide64Regs)
 enum BatchWalk { kBinary, kWide32, kWide64 };
 template <int KIND, int WALK, bool LOCAL, uint32_t LCAP>
 constexpr auto batch_fn() {
-  if constexpr (WALK == kWide32)
+  if constexpr (WALK == kWide32 && KIND != kCylinders)
     return trace_batch_wide_kernel<KIND, LOCAL, LCAP>;
   else if constexpr (WALK == kWide64 && LOCAL && KIND != kCylinders)
     return trace_batch_wide64_kernel<KIND, LCAP>;
