@@ -550,11 +550,11 @@ def run_ours(args):
             "step_ms_min_max": [min(res["mixed"]["step_ms"]), max(res["mixed"]["step_ms"])]}
     # one traversal kernel per primitive kind present, per step
     n_passes = sum(1 for k in wl.scene.order if len(next(iter(getattr(wl.scene, k).values()))))
-    # kernels per call: one per kind present; the triangle, sphere and plane passes add one before
-    # the wide walk, for the rays it leaves out, and one after it, for those it hands on
+    # kernels per call: one per kind present; the triangle, sphere and plane passes add one after
+    # the wide walk, for the rays it hands on
     n_wide = sum(1 for k in wl.scene.order
                  if k != "cylinders" and len(next(iter(getattr(wl.scene, k).values()))))
-    launches_per_call = {"fp64": n_passes + 2 * n_wide, "mixed": n_passes + 2 * n_wide}
+    launches_per_call = {"fp64": n_passes + n_wide, "mixed": n_passes + n_wide}
 
     # roofline of the primary path's traversal kernels.  Algorithmic bytes from the walk's own work
     # counts (untimed counting run): ray I/O + 128 B per wide node (cylinders: 64 B per box test,
@@ -824,8 +824,8 @@ def run_adjoint(args):
                        "l2": "flushed between timed steps (256 MiB write)"},
             "adjoint_ms_per_step": adj_ms / args.steps, "hit_fraction": hit_frac,
             "e2e": e2e,
-            # two kind passes of three kernels, the ray and face adjoint kernels
-            "gpu_launches": args.steps * 8,
+            # two kind passes of two kernels, the ray and face adjoint kernels
+            "gpu_launches": args.steps * 6,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "peak_source": peak_src},
             "cpu_baseline": cpu, "clocks": clocks}), flush=True)

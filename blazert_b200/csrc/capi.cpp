@@ -649,10 +649,10 @@ static int staged_wait_result(bzr_scene *s, int rc) {
 // [normal], [prim], [geom], [hit]; each piece 256-byte aligned; then a flag.  The kernel of
 // trace_small.cu reads and writes that block itself and raises the flag at its end, which the
 // host watches: the launch is the call's only GPU operation.  (With a memset, two copies and a
-// poll of the stream around the kernels one ray took 51 us, now 39, both from
-// Python; 3,001 rays through three kinds 231 -> 118 us.)  Where that kernel does not apply (counting, a coherence sort, a
-// shared-memory stack) a device block mirrors the pinned one: one copy in, the kind passes on a
-// grid sized to the batch, one copy out.
+// poll of the stream around the kernels of each kind one ray took 52 us, now 36, both from Python;
+// 3,001 rays through three kinds 305 -> 112 us.)  Where that kernel does not apply (counting, a
+// coherence sort, a shared-memory stack) a device block mirrors the pinned one: one copy in, the
+// kind passes on a grid sized to the batch, one copy out.
 static int run_small(bzr_scene *s, size_t n, const double *org, const double *dir,
                      const double *tmin, const double *tmax, double *t, double *uv, double *normal,
                      uint32_t *prim, uint32_t *geom, uint8_t *hit, int mode, bzr::RayIO io,
@@ -795,7 +795,7 @@ static int wait_event(cudaEvent_t ev, int timeout_ms) {
 // block, one copy takes it to the device, the kernels run, one copy brings the results back and
 // the threads unpack them, while the next chunks are on their way.  What is left is the host's
 // own copying (and the page faults of fresh result arrays), which the threads share.
-// 1,048,576 rays through three kinds, plain numpy arrays: 18.1 -> 5.5 ms.
+// 1,048,576 rays through three kinds, plain numpy arrays: 18.1 -> 6.2 ms.
 // Arrays that the caller pinned go straight between their place and the device, beside the block.
 // A block: the pageable ones of org, dir, [tmin], [tmax], the error word, the pageable ones of
 // the requested outputs; on the device only, the pinned inputs and outputs after them, and t when

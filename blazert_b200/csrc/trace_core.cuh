@@ -770,10 +770,10 @@ BZR_HD RayW make_ray_f(const Ray &r, const RayW *) {
 // decision that accepts a hit are the binary walk's, in FP64, so the results are its bits by the
 // argument above; the quantised boxes only skip subtrees that the FP64 test of their exact boxes
 // skips.
-// B200, FP64 mode, device arrays: 8.4M bounce rays on that terrain 7,822 -> 4,606 us; 1M rays
-// through 10,000 spheres, 1,000 cylinders and 100 planes 1,711 -> 1,387 us; 512 x 512 rays on a
-// 5,120-triangle sphere 117 -> 94 us.  It runs at 1.10 times the FP32 walk's time on the
-// terrain: 48 FP64 multiply-adds per node, which the FP64 pipe has room for.
+// B200, FP64 mode, device arrays, when this walk came: 8.4M bounce rays on that terrain 7,822 ->
+// 4,606 us; 1M rays through 10,000 spheres, 1,000 cylinders and 100 planes 1,711 -> 1,387 us;
+// 512 x 512 rays on a 5,120-triangle sphere 117 -> 94 us.  It runs at 1.09 times the FP32 walk's
+// time on the terrain: 48 FP64 multiply-adds per node, which the FP64 pipe has room for.
 //
 // Two things end a wide walk without a result; such a ray is traced again by the binary walk
 // (kRedoLeaf, and rays whose f.ok is false before they start):

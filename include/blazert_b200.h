@@ -246,8 +246,8 @@ int bzr_scene_check(const bzr_scene *scene, void *stream, int timeout_ms, uint32
 #define BZR_TUNE_BLOCK 3
 #define BZR_TUNE_STACK 4
 #define BZR_TUNE_CHUNK 5
-/* Host-array calls from pinned memory (and of less than 196,608 rays from ordinary memory): the
- * batch is split into at most this many chunks (1 to 32, default 8) of
+/* Host-array calls from pinned memory (or with ordinary memory for tmin and tmax alone, or of less
+ * than 196,608 rays): the batch is split into at most this many chunks (1 to 32, default 8) of
  * at least BZR_TUNE_HOST_MIN_CHUNK rays (default 131,072), pipelined as copies in, kernels and
  * copies out. */
 #define BZR_TUNE_HOST_CHUNKS 6
