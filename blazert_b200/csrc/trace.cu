@@ -143,12 +143,12 @@ struct Rest {
 // the slowest: the middle row of an image of odd height has a zero direction component, and along a
 // plane of box bounds the reference's 0 * inf accepts thousands of boxes.  Traced after the wide
 // walk instead, they added their whole time to it: 541,501 pixels of a 20,480-triangle sphere
-// 637 us, now 441; without that row 166.  (As a first phase, or a last one, of every block they
+// 637 us, now 361; without that row 166.  (As a first phase, or a last one, of every block they
 // cost the walk its registers: 8.4M bounce rays on a terrain 4,420 -> 4,560 to 4,850 us; a look
 // through those takes about 10.  As a kernel of its own, which the wide one must run beside to gain
-// anything, they have more registers, 420 us for that image, but the wide kernel then reads what
-// earlier kernels wrote without a wait of its own; an acquire in its place empties the SM's L1
-// under the walks, 3 to 13 us a pass at 131,072 rays.)
+// anything, they have more registers, 420 us for that image where these then took 441, but the wide
+// kernel then reads what earlier kernels wrote without a wait of its own; an acquire in its place
+// empties the SM's L1 under the walks, 3 to 13 us a pass at 131,072 rays.)
 constexpr uint32_t kScan = 8;  // runs of 32 rays a warp looks at together: independent loads
 
 // Whether the wide walk covers hardly any ray of a large batch (an orthographic camera along an
@@ -200,8 +200,12 @@ __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const Ra
   if (covers_hardly_any<KIND, F>(io)) return;
   const uint32_t warps = uint32_t(io.out_blocks) * (blockDim.x >> 5);
   const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  // runs of 32 rays, dealt to the warps in turn (left-out rays tend to lie together), kScan runs
-  // looked at together
+  // Runs of 32 rays, dealt to the warps in turn (left-out rays tend to lie together), kScan runs
+  // looked at together.  On a mesh a run is four pieces of 8 rays from the batch's four quarters, as
+  // the slow rays of an image's middle row take the longer the more of them a warp has: 541,501
+  // pixels of a 20,480-triangle sphere 445 us in whole runs, 361 so (mixed 480 and 387).  Elsewhere
+  // rays rarely run along boxes, and whole runs are the better by 3 to 6 % where all are left out.
+  constexpr uint32_t kPiece = KIND == kMesh ? 8 : 32;
   uint64_t run = warp;
   const uint64_t runs = (uint64_t(io.n) + 31) / 32;
   unsigned found[kScan] = {};  // warp-uniform: the left-out rays of the runs, not yet taken
@@ -211,6 +215,9 @@ __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const Ra
   Ray r;
   KState st;
   Trav tv;
+  auto ray_of = [&](uint64_t k, uint32_t b) {
+    return (k + uint64_t(b / kPiece) * runs) * kPiece + b % kPiece;
+  };
   auto any_found = [&] {
     unsigned m = 0;
 #pragma unroll
@@ -222,9 +229,9 @@ __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const Ra
     while (idle && run < runs && !any_found()) {
 #pragma unroll
       for (uint32_t j = 0; j < kScan; ++j) {
-        const uint64_t idx = (run + uint64_t(j) * warps) * 32 + lane;
+        const uint64_t idx = ray_of(run + uint64_t(j) * warps, lane);
         bool out = false;
-        if (idx < io.n) {
+        if (run + uint64_t(j) * warps < runs && idx < io.n) {
           const double w[3] = {io.dir[3 * idx], io.dir[3 * idx + 1], io.dir[3 * idx + 2]};
           out = left_out(w, io.tmin ? io.tmin[idx] : 0.0, io.tmax ? io.tmax[idx] : kDblMax,
                          static_cast<const F *>(nullptr));
@@ -243,7 +250,7 @@ __device__ __forceinline__ void trace_left_out_body(const SceneView &S, const Ra
         if (!active && !got && rank < have) {
           unsigned m = found[j];
           for (uint32_t k = 0; k < rank; ++k) m &= m - 1;
-          i = uint32_t((at + uint64_t(j) * warps) * 32) + unsigned(__ffs(m)) - 1u;
+          i = uint32_t(ray_of(at + uint64_t(j) * warps, unsigned(__ffs(m)) - 1u));
           got = true;
         }
         if (!got) rank -= have < rank ? have : rank;
