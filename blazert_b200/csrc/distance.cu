@@ -40,11 +40,11 @@ __global__ void __launch_bounds__(kDistanceThreads)
 }
 
 // Cylinders: the ellipse search takes 8 Newton steps per point on average and seldom more than 25
-// (random points, with ellipse_search_step's cycle rule; the limit is kSearchSteps = 100), so a warp of 32 fixed queries would idle lanes while its
-// slowest one iterates.  Here each warp owns a contiguous range of queries and refills idle
-// lanes from it: a trip of the loop gives new queries to the idle lanes (their decisions before
-// the search, cylinder_setup) and one search step to the lanes in a search, all four sectors
-// in the same instructions.
+// (random points, with ellipse_search_step's cycle rule; the limit is kSearchSteps = 100), so a
+// warp of 32 fixed queries would idle lanes while its slowest one iterates.  Here each warp owns a
+// contiguous range of queries and refills idle lanes from it: a trip of the loop gives new queries
+// to the idle lanes (their decisions before the search, cylinder_setup) and one search step to the
+// lanes in a search, all four sectors in the same instructions.
 //
 // A refill costs about two search steps whatever the number of lanes it fills, so it waits
 // until kRefillLanes are idle, and one wave of kCylinderBlocks resident blocks per SM gives

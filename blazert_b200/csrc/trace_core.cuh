@@ -665,13 +665,13 @@ BZR_HD bool traverse(const KindView &K, const Ray &r, KState &st, const Stack &s
 // The bound follows the ray's own magnitudes on each axis: an axis whose direction component
 // is tiny has large distances and a large E, but those distances rarely decide the entry or
 // the exit.  Rays with a zero, non-finite, large (> 2^40) or small (< 2^-100) inverse direction
-// component, an origin component beyond 1e18, or a non-finite or huge tmin or a NaN tmax, take the FP64
-// traversal.  Then every FP32 value of the test is finite: node coordinates are within 1e18
-// (the builder's limit), so 2^e <= 2^54, |A| <= 2^94, 2^23 |A| <= 2^117, |B| <= 2^101, and
-// every distance and difference stays below 2^121.  And inv_f is a normal number, rounded within
-// 2^-24 of the FP64 inverse as the bound has it: a denormal one (a raw direction beyond 2^126) has
-// fewer bits and loses hits where coordinates are large (1e9 and more).  A and B may still be
-// denormal; their absolute errors of 2^-150, times 2^23 at most, are within the 1e-37.
+// component, an origin component beyond 1e18, or a non-finite or huge tmin or a NaN tmax, take the
+// FP64 traversal.  Then every FP32 value of the test is finite: node coordinates are within 1e18
+// (the builder's limit), so 2^e <= 2^54, |A| <= 2^94, 2^23 |A| <= 2^117, |B| <= 2^101, and every
+// distance and difference stays below 2^121.  And inv_f is a normal number, rounded within 2^-24 of
+// the FP64 inverse as the bound has it: a denormal one (a raw direction beyond 2^126) has fewer
+// bits and loses hits where coordinates are large (1e9 and more).  A and B may still be denormal;
+// their absolute errors of 2^-150, times 2^23 at most, are within the 1e-37.
 struct RayW {
   using Bound = float;
   float o_hi[3], o_lo[3], inv[3];
